@@ -33,7 +33,7 @@ EXPORTED_SYMBOLS = [
     "b200ml_cast", "b200ml_conv2d", "b200ml_se_gate", "b200ml_attention_f16", "b200ml_strided_copy", "b200ml_gather",
     "b200ml_where", "b200ml_compare", "b200ml_maxpool2d", "b200ml_wait_probe", "b200ml_strided_copy_parts",
     "b200ml_peer_allgather", "b200ml_ipc_export", "b200ml_ipc_open", "b200ml_ipc_close",
-    "b200ml_conv_prepack_bytes", "b200ml_conv_prepack",
+    "b200ml_conv_prepack_bytes", "b200ml_conv_prepack", "b200ml_plan_create", "b200ml_plan_destroy", "b200ml_plan_run",
 ]
 
 
@@ -159,6 +159,9 @@ def load_library(path=None):
         lib.b200ml_ipc_export.argtypes = [vp, vp, vp, i64p]
         lib.b200ml_ipc_open.argtypes = [vp, vp, c_i64, ctypes.POINTER(vp)]
         lib.b200ml_ipc_close.argtypes = [vp, vp, c_i64]
+        lib.b200ml_plan_create.argtypes = [c_i32, i32p, i64p, ctypes.c_char_p, c_i64, c_i32, i64p, c_i32, ctypes.POINTER(vp)]
+        lib.b200ml_plan_destroy.argtypes = [vp]
+        lib.b200ml_plan_run.argtypes = [vp, vp, vp, c_i32, vp]
         for name in EXPORTED_SYMBOLS:
             fn = getattr(lib, name)
             if name not in ("b200ml_last_error", "b200ml_launch_count", "b200ml_ctx_workspace_bytes", "b200ml_conv_prepack_bytes"):

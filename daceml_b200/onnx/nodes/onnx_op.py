@@ -38,6 +38,9 @@ def parse_variadic_param(param):
     return split[0], int(split[1])
 
 
+_BUILTIN_IMPLEMENTATIONS = tuple("daceml_b200.onnx.op_implementations." + m for m in ("b200_implementations", "indexing_implementations"))
+
+
 class Expansion:
     """Base of the per-(op, implementation) expansion classes, like ``ExpandTransformation``."""
     environments = []
@@ -47,7 +50,11 @@ class Expansion:
     def expansion(cls, node, state, sdfg, **kwargs):
         node.validate(sdfg, state)
         if cls.forward_impl.forward_can_be_applied(node, state, sdfg):
-            return cls.forward_impl.forward(node, state, sdfg, **kwargs)
+            result = cls.forward_impl.forward(node, state, sdfg, **kwargs)
+            # this library's own implementations only make C ABI calls that depend on shapes and attributes
+            if isinstance(result, sd.KernelTasklet) and cls.forward_impl.forward.__module__ in _BUILTIN_IMPLEMENTATIONS:
+                result.recordable = True
+            return result
         raise NotImplementedError(
             'Library node "{}": implementation "{}" cannot be applied (forward_can_be_applied returned False) '
             'and this build has no ONNX Runtime fallback'.format(node.label, cls.__name__))

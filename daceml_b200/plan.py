@@ -1,0 +1,136 @@
+"""Launch plans: the calls of a compiled SDFG recorded once and run natively (``csrc/plan.cu``).
+
+The reference compiles an SDFG into a library whose one entry point takes the tensors' addresses
+(``daceml/torch/dispatchers/common.py:34-76``).  Here the tasklets of a compiled SDFG are run once with a recording
+context in the place of the real one: every call into the C ABI is written down instead of made, and addresses that
+lie inside an input or output of the SDFG become places to fill in.  Running the plan is then one foreign-function call
+with the addresses of this call's tensors, whatever the number of launches.
+"""
+import ctypes
+import struct
+
+import torch
+
+from . import lib as L
+
+# entry points in the order of the PlanOp enumeration; 'i' integer, 'f' float, 'p' address, 's' structure by
+# reference, 'a' array of numbers, 'q' array of addresses (the arguments between the context and the stream)
+_CALLS = [
+    ("b200ml_gemm", "s"), ("b200ml_softmax", "ipppiiifi"), ("b200ml_layernorm", "ippppppiif"), ("b200ml_reduce", "iippiii"),
+    ("b200ml_unary", "iippiff"), ("b200ml_binary", "iipppiaaa"), ("b200ml_bias_act", "ippppiii"), ("b200ml_transpose", "ippiaa"),
+    ("b200ml_cast", "iippi"), ("b200ml_conv2d", "s"), ("b200ml_se_gate", "ippppppiii"), ("b200ml_attention_f16", "s"),
+    ("b200ml_strided_copy", "ippiaaa"), ("b200ml_strided_copy_parts", "iiqqiaaa"), ("b200ml_gather", "ipppiiii"),
+    ("b200ml_where", "ippppiaaaa"), ("b200ml_compare", "iipppiaaa"), ("b200ml_maxpool2d", "ippiiiiiiiiiii"),
+]
+
+
+class NotRecordable(Exception):
+    """A tasklet did something a plan cannot hold."""
+
+
+def _value(x):
+    return 0 if x is None else int(getattr(x, "value", x) or 0)
+
+
+class _RecorderLib:
+    """Stands in for the loaded library while tasklets are recorded."""
+
+    def __init__(self):
+        self.ops, self.offsets, self.blob, self.pointers = [], [], bytearray(), []
+        for code, (name, kinds) in enumerate(_CALLS):
+            setattr(self, name, self._entry(code, kinds))
+
+    def __getattr__(self, name):
+        raise NotRecordable(name)
+
+    def _append(self, data, pointer_offsets=()):
+        at = len(self.blob)
+        self.blob += bytes(data)
+        self.blob += bytes(-len(self.blob) % 8)
+        self.pointers += [at + o for o in pointer_offsets]
+        return at
+
+    def _entry(self, code, kinds):
+        def call(handle, *args):
+            if len(args) != len(kinds) + 1:  # the stream is last
+                raise NotRecordable("argument count")
+            self.ops.append(code)
+            at = len(self.blob)
+            self.offsets.append(at)
+            self.blob += bytes(8 * len(kinds))
+            for i, (kind, x) in enumerate(zip(kinds, args)):
+                if kind == "i":
+                    word = struct.pack("q", _value(x))
+                elif kind == "f":
+                    word = struct.pack("d", float(x))
+                elif kind == "p":
+                    word = struct.pack("Q", _value(x))
+                    self.pointers.append(at + 8 * i)
+                elif kind == "s":
+                    s = x._obj  # ctypes.byref(structure)
+                    fields = [getattr(type(s), n).offset for n, t in s._fields_ if t is ctypes.c_void_p]
+                    word = struct.pack("q", self._append(s, fields))
+                elif kind == "q":
+                    word = struct.pack("q", self._append(x, range(0, ctypes.sizeof(x), 8)))
+                else:
+                    word = struct.pack("q", self._append(x))
+                self.blob[at + 8 * i:at + 8 * i + 8] = word
+            return L.OK
+
+        return call
+
+
+class _RecordingContext:
+    def __init__(self, device):
+        self.lib, self.device, self.handle = _RecorderLib(), device, ctypes.c_void_p()
+
+
+class LaunchPlan:
+    """The native plan of ``tasklets`` (``(tasklet, ins, outs)`` triples with array names as values).
+
+    ``bound`` maps every array name to a tensor; those named in ``io`` (in this order) and their views are the ones a run
+    replaces.  The addresses of the ``fixed`` tensors (constants, transients) are part of the plan, which keeps them alive
+    together with whatever the tasklets hold."""
+
+    def __init__(self, tasklets, bound, io, fixed, device):
+        rec = _RecordingContext(device.index)
+        with L.use_context(rec):
+            for tasklet, ins, outs in tasklets:
+                if not tasklet.recordable:
+                    raise NotRecordable(tasklet.label)
+                tasklet.fn({c: bound[a] for c, a in ins.items()}, {c: bound[a] for c, a in outs.items()})
+        r = rec.lib
+        ranges = [(bound[n].data_ptr(), bound[n].data_ptr() + bound[n].numel() * bound[n].element_size(), s) for s, n in enumerate(io)]
+        if any(lo == 0 or lo == hi for lo, hi, _ in ranges):
+            raise NotRecordable("an empty tensor")
+        patches = []
+        for at in r.pointers:
+            addr = struct.unpack_from("Q", r.blob, at)[0]
+            for lo, hi, slot in ranges:
+                if lo <= addr < hi:
+                    patches += [at, slot, addr - lo]
+        n = len(r.ops)
+        self.lib = L.load_library()
+        self.n_slots = len(io)
+        self.keep = (list(fixed), [t for t, _, _ in tasklets])
+        handle = ctypes.c_void_p()
+        blob = bytes(r.blob) or b"\0" * 8
+        L.check(self.lib.b200ml_plan_create(n, (ctypes.c_int32 * n)(*r.ops), (ctypes.c_int64 * n)(*r.offsets), blob, len(blob),
+                                            len(patches) // 3, (ctypes.c_int64 * len(patches))(*patches), len(io), ctypes.byref(handle)))
+        self.handle = handle
+        self._slots = ctypes.c_void_p * len(io)
+        self._run = self.lib.b200ml_plan_run
+        self._device = device
+        self._index = device.index
+
+    def __del__(self):
+        handle, self.handle = getattr(self, "handle", None), None
+        if handle:
+            self.lib.b200ml_plan_destroy(handle)
+
+    def __call__(self, *addresses):
+        """Enqueues the plan on the current stream; ``addresses``: one ``data_ptr()`` per name of ``io``."""
+        rc = self._run(self.handle, L.get_context(self._device).handle, self._slots(*addresses), self.n_slots,
+                       torch._C._cuda_getCurrentRawStream(self._index))
+        if rc:
+            L.check(rc)

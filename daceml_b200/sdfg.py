@@ -85,6 +85,9 @@ class KernelTasklet(Node):
         self.label = label
         self.fn = fn
         self.kernels = tuple(kernels)
+        # whether ``fn`` does nothing but call the C ABI, with arguments that depend on its tensors' addresses and shapes
+        # only: such a tasklet can be recorded once and run from a native launch plan
+        self.recordable = False
 
     def __repr__(self):
         return f"KernelTasklet({self.label})"
@@ -187,13 +190,34 @@ class SDFGState:
         return order
 
 
+class _Constants(dict):
+    """Constants by name; ``version`` changes with every replacement, so that a recorded launch plan can tell."""
+    version = 0
+
+    def __setitem__(self, key, value):
+        self.version += 1
+        super().__setitem__(key, value)
+
+    def __delitem__(self, key):
+        self.version += 1
+        super().__delitem__(key)
+
+    def pop(self, *args):
+        self.version += 1
+        return super().pop(*args)
+
+    def update(self, *args, **kwargs):
+        self.version += 1
+        super().update(*args, **kwargs)
+
+
 class SDFG:
     def __init__(self, name):
         self.name = name
         self.arrays: Dict[str, Data] = {}
         self._states: List[SDFGState] = []
         # constants bound at build time (weights), name -> tensor; the importer's ``weights`` dict
-        self.constants: Dict[str, torch.Tensor] = {}
+        self.constants: Dict[str, torch.Tensor] = _Constants()
 
     def add_array(self, name, shape, dtype, transient=False):
         if name in self.arrays:
@@ -263,7 +287,8 @@ class CompiledSDFG:
 
     ``__call__`` binds caller tensors by array name (numpy arrays are staged through the GPU and
     copied back, torch CUDA tensors are used in place), allocates ``__return*`` arrays if the
-    caller did not pass them, and enqueues every tasklet on the current CUDA stream."""
+    caller did not pass them, and enqueues every tasklet on the current CUDA stream: through the native launch plan
+    from the second call on, where the tasklets and arguments allow it."""
 
     def __init__(self, sdfg: SDFG, device: Optional[torch.device] = None):
         self.sdfg = sdfg
@@ -277,6 +302,10 @@ class CompiledSDFG:
                 outs = {e.src_conn: e.data.data for e in st.out_edges(n)}
                 self.plan.append((n, ins, outs))
         self._transients = {}
+        self._calls = 0
+        self._native = None  # the recorded launch plan; False when there cannot be one
+        self._native_version = -1
+        self._io = None
         if device is not None or torch.cuda.is_available():
             self.allocate_transients()
 
@@ -295,6 +324,82 @@ class CompiledSDFG:
             self.device = torch.device("cuda", torch.cuda.current_device())
         return self.device
 
+    def _constant(self, name):
+        """The constant's tensor on this SDFG's device (moved there on first use)."""
+        t = self.sdfg.constants[name]
+        if not t.is_cuda:
+            t = self.sdfg.constants[name] = t.to(self._device()).contiguous()
+        return t
+
+    def io_names(self):
+        """The arrays a caller passes or gets back: inputs and ``__return*`` outputs."""
+        arrays, consts = self.sdfg.arrays, self.sdfg.constants
+        return [n for n, d in arrays.items() if not d.transient and d.view_of is None and n not in consts]
+
+    def launch_plan(self, tensors=None):
+        """The native launch plan of this SDFG over :meth:`io_names` (see :mod:`daceml_b200.plan`), recorded on first use
+        and again after a constant was replaced; None when a tasklet runs code of its own.  ``tensors`` may hold inputs to
+        record with (only their addresses are looked at), which saves allocating some."""
+        if self._native is False:
+            return None
+        if self._native is None or self._native_version != self.sdfg.constants.version:
+            from daceml_b200.plan import LaunchPlan, NotRecordable
+            self._native = False
+            if NVTX_RANGES or not all(t.recordable for t, _, _ in self.plan):
+                return None
+            dev = self._device()
+            self.allocate_transients()
+            io = self.io_names()
+            fixed = {n: self._constant(n) for n in list(self.sdfg.constants)}
+            fixed.update(self._transients)
+            bound = dict(fixed)
+            for n in io:
+                desc, t = self.sdfg.arrays[n], (tensors or {}).get(n)
+                if t is None or t.device != dev or t.shape != desc.shape or t.dtype != desc.dtype or not t.is_contiguous():
+                    t = torch.empty(desc.shape, dtype=desc.dtype, device=dev)
+                bound[n] = t
+            for n, desc in self.sdfg.arrays.items():
+                if n not in bound:
+                    bound[n] = bound[self.sdfg.root_of(n)].view(desc.shape)
+            try:
+                self._native = LaunchPlan(self.plan, bound, io, fixed.values(), dev)
+                self._native_version, self._io = self.sdfg.constants.version, io
+            except NotRecordable:
+                return None
+        return self._native
+
+    def _run_plan(self, plan, kwargs):
+        """One run of the launch plan on ``kwargs``; ``NotImplemented`` when the arguments need the general path (host
+        data, other layouts, constants or transients passed by the caller, errors to report)."""
+        index, arrays = self.device.index, self.sdfg.arrays
+        addresses, returns, given = [], {}, 0
+        for name in self._io:
+            desc, t = arrays[name], kwargs.get(name)
+            if t is None:
+                if not name.startswith("__return"):
+                    return NotImplemented
+                t = returns[name] = torch.empty(desc.shape, dtype=desc.dtype, device=self.device)
+            else:
+                given += 1
+                if (not isinstance(t, torch.Tensor) or t.get_device() != index or t.shape != desc.shape or t.dtype != desc.dtype
+                        or not t.is_contiguous()):
+                    return NotImplemented
+            addresses.append(t.data_ptr())
+        if given != len(kwargs):
+            return NotImplemented
+        plan(*addresses)
+        return self._returned(returns)
+
+    @staticmethod
+    def _returned(named):
+        """The ``__return*`` tensors as the caller gets them."""
+        if not named:
+            return None
+        # '__return', '__return_0', ... '__return_10': by number, not by string ('__return_10' < '__return_2')
+        order = sorted(named, key=lambda n: (int(n.rsplit("_", 1)[1]) if n.rsplit("_", 1)[1].isdigit() else -1, n))
+        outs = [named[n] for n in order]
+        return outs[0] if len(outs) == 1 else tuple(outs)
+
     def kernel_names(self):
         return [k for t, _, _ in self.plan for k in t.kernels]
 
@@ -311,6 +416,13 @@ class CompiledSDFG:
 
     def __call__(self, **kwargs):
         dev = self._device()
+        self._calls += 1
+        if self._calls > 1:  # a graph that runs once (an eager operator call) is not worth recording
+            plan = self.launch_plan()
+            if plan is not None:
+                result = self._run_plan(plan, kwargs)
+                if result is not NotImplemented:
+                    return result
         bound: Dict[str, torch.Tensor] = {}
         copy_back = []
         for name, val in kwargs.items():
@@ -331,11 +443,9 @@ class CompiledSDFG:
             if tuple(t.shape) != desc.shape or t.dtype != desc.dtype:
                 raise ValueError(f"argument '{name}' is {tuple(t.shape)} {t.dtype}, expected {desc.shape} {desc.dtype}")
             bound[name] = t
-        for name, t in self.sdfg.constants.items():
+        for name in list(self.sdfg.constants):
             if name not in bound:
-                if not t.is_cuda:
-                    t = self.sdfg.constants[name] = t.to(dev).contiguous()
-                bound[name] = t
+                bound[name] = self._constant(name)
         returns = []
         views = []
         for name, desc in self.sdfg.arrays.items():
@@ -377,10 +487,7 @@ class CompiledSDFG:
                 host[...] = devt.cpu().numpy()
             else:
                 host.copy_(devt)
-        if not returns:
-            return None
-        # '__return', '__return_0', ... '__return_10': by number, not by string ('__return_10' < '__return_2')
-        outs = [bound[n] for n in sorted(returns, key=lambda n: (int(n.rsplit("_", 1)[1]) if n.rsplit("_", 1)[1].isdigit() else -1, n))]
+        named = {n: bound[n] for n in returns}
         if any(isinstance(v, np.ndarray) for v in kwargs.values()):
-            outs = [o.cpu().numpy() for o in outs]
-        return outs[0] if len(outs) == 1 else tuple(outs)
+            named = {n: o.cpu().numpy() for n, o in named.items()}
+        return self._returned(named)

@@ -195,21 +195,27 @@ class DaceModule(nn.Module):
         input_names = list(self.sdfg.arg_names)
         output_names = list(dace_model.outputs)
 
-        def run(*args):
+        arrays, debug = self.sdfg.arrays, self.debug_transients
+
+        def run_general(*args):
             if len(args) != len(input_names):
                 raise ValueError("Expected {} arguments, got {}".format(len(input_names), len(args)))
             kwargs = dict(zip(input_names, args))
             outs = {}
-            if len(output_names) != 1 or output_names[0] != "__return" or self.debug_transients:
+            if len(output_names) != 1 or output_names[0] != "__return" or debug:
                 dev = compiled._device()
                 for name in output_names:
-                    desc = self.sdfg.arrays[name]
+                    desc = arrays[name]
                     outs[name] = torch.empty(desc.shape, dtype=desc.dtype, device=dev)
             result = compiled(**kwargs, **outs)
             if outs:
                 vals = tuple(outs[n] for n in output_names)
                 return vals[0] if len(vals) == 1 else vals
             return result
+
+        run = run_general
+        if torch.cuda.is_available() and not debug:
+            run = self._planned_call(compiled, input_names, output_names, run_general, dummy_inputs) or run_general
 
         if not self.cuda_graph:
             return self._as_torch_op(run, input_names, output_names)
@@ -239,6 +245,37 @@ class DaceModule(nn.Module):
         self.static_inputs = static_in
         return self._as_torch_op(replay, input_names, output_names)
 
+    @staticmethod
+    def _planned_call(compiled, input_names, output_names, general, example):
+        """The module as one run of the compiled SDFG's launch plan: checks the arguments, allocates the outputs, passes
+        the addresses.  ``general`` serves what the plan does not take (host or strided tensors, errors to report)."""
+        tensors = {n: t for n, t in zip(input_names, example) if isinstance(t, torch.Tensor)}
+        plan = compiled.launch_plan(tensors if len({t.data_ptr() for t in tensors.values()}) == len(tensors) else None)
+        if plan is None or sorted(compiled.io_names()) != sorted(input_names + output_names):
+            return None
+        arrays, constants = compiled.sdfg.arrays, compiled.sdfg.constants
+        specs = [(torch.Size(arrays[n].shape), arrays[n].dtype) for n in input_names]
+        out_specs = [(torch.Size(arrays[n].shape), arrays[n].dtype) for n in output_names]
+        order = [(input_names + output_names).index(n) for n in compiled.io_names()]
+        in_order = order == list(range(len(order)))
+        device, version, n_in = compiled.device, constants.version, len(specs)
+        index, single, empty, tensor_types = device.index, len(out_specs) == 1, torch.empty, (torch.Tensor, nn.Parameter)
+
+        def run(*args):
+            if len(args) != n_in or constants.version != version:
+                return general(*args)
+            addresses = []
+            for a, (shape, dtype) in zip(args, specs):
+                if type(a) not in tensor_types or a.get_device() != index or a.dtype is not dtype or a.shape != shape or not a.is_contiguous():
+                    return general(*args)
+                addresses.append(a.data_ptr())
+            outs = [empty(shape, dtype=dtype, device=device) for shape, dtype in out_specs]
+            addresses += [o.data_ptr() for o in outs]
+            plan(*(addresses if in_order else [addresses[i] for i in order]))
+            return outs[0] if single else tuple(outs)
+
+        return run
+
     def _as_torch_op(self, function, input_names, output_names):
         """With ``compile_torch_extension`` (the default, as in the reference) the module is called through a registered
         torch operator, ``torch.ops.daceml_<sdfg_name>.<sdfg_name>(handle, *inputs)``; otherwise directly."""
@@ -255,6 +292,11 @@ class DaceModule(nn.Module):
         self.torch_op, self.torch_op_handle = op, handle
 
         def call(*args):
+            # Called from plain Python the operator is only a detour (its dispatch costs more than a small module's
+            # launches); what looks at operators - tracing, torch.compile, a mode, a tensor subclass - gets it.
+            if not (torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack()
+                    or torch._C._is_torch_function_mode_enabled()) and all(type(a) is torch.Tensor for a in args):
+                return function(*args)
             if not all(isinstance(a, torch.Tensor) and a.is_cuda for a in args):
                 return function(*args)  # host tensors are staged by the compiled SDFG itself
             result = op(handle, *args)

@@ -401,6 +401,25 @@ typedef struct {
  * around it (pure_implementations.py:111-216, 309-326). */
 int b200ml_attention_f16(b200ml_ctx* ctx, const b200ml_attention_params* p, b200ml_stream stream);
 
+/* ------------------------------------------------------------------------- */
+/* Launch plans                                                               */
+/* ------------------------------------------------------------------------- */
+
+/* The calls of a compiled graph as one object: what the reference's generated SDFG library is to its dispatcher
+ * (daceml/torch/dispatchers/common.py:34-76).  `ops` names the entry point of each call (the order of the PlanOp
+ * enumeration in csrc/plan.cu), `offsets` where its argument words start in `blob`: one 64-bit word per argument between
+ * the context and the stream (integers and addresses as they are, floats as a double); a structure or an array is stored in
+ * the blob and its word holds the byte offset.  `patches` are triples (byte offset of an address in the blob, slot, bytes
+ * to add): a run writes the address of slots[slot] there.  A plan owns a copy of its blob; the memory the other addresses
+ * name belongs to the caller. */
+typedef struct b200ml_plan b200ml_plan;
+int b200ml_plan_create(int32_t n_calls, const int32_t* ops, const int64_t* offsets, const void* blob, int64_t blob_bytes,
+                       int32_t n_patches, const int64_t* patches, int32_t n_slots, b200ml_plan** out);
+int b200ml_plan_destroy(b200ml_plan* plan);
+/* Enqueues every call on `stream`; stops at the first that fails and returns its status.  Any number of threads may run one
+ * plan at a time (the scratch of the context and the memory the plan's addresses name still serve one run on the GPU). */
+int b200ml_plan_run(const b200ml_plan* plan, b200ml_ctx* ctx, void* const* slots, int32_t n_slots, b200ml_stream stream);
+
 #ifdef __cplusplus
 }
 #endif

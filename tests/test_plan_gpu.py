@@ -1,0 +1,74 @@
+"""Launch plans: a graph run natively gives the bits the tasklets give one by one, for tensors it was not recorded on."""
+import copy
+
+import pytest
+import torch
+import torch.nn as nn
+
+from daceml_b200 import lib as L
+from daceml_b200.torch import DaceModule
+from models import LeNet, MBConv, TinyBert
+
+pytestmark = pytest.mark.gpu
+
+
+class Mixed(nn.Module):
+    """Views of inputs and outputs, several parts per launch, index and mask operands."""
+
+    def forward(self, x, ids):
+        a, b = torch.split(x, [3, 5], dim=1)
+        t = torch.cat([b, a], dim=1).transpose(0, 1)
+        y = torch.where(t > 0, t * 2.0, torch.exp(t))
+        return y.reshape(-1, 4), y[:, :2].sum(dim=0), x[ids], torch.softmax(x, dim=1)
+
+
+def _case(name):
+    if name == "mixed":
+        return Mixed(), lambda: (torch.randn(4, 8), torch.tensor([2, 0, 3]))
+    if name == "lenet":
+        return LeNet(), lambda: (torch.rand(3, 1, 32, 32), )
+    if name == "mbconv":
+        return MBConv(8, 16, 2), lambda: (torch.randn(2, 8, 9, 11), )
+    return TinyBert(layers=1), lambda: (torch.randint(0, 1000, (2, 13)), (torch.rand(2, 13) > 0.2).long())
+
+
+@pytest.mark.parametrize("name", ["mixed", "lenet", "mbconv", "bert"])
+def test_plan_gives_the_bits_of_the_tasklets(name):
+    torch.manual_seed(0)
+    net, inputs = _case(name)
+    net = net.eval()
+    module = DaceModule(copy.deepcopy(net), dummy_inputs=inputs())
+    compiled = module.compiled_function
+    assert compiled.launch_plan() is not None
+    for _ in range(3):
+        args = tuple(t.cuda() for t in inputs())
+        got = module(*args)
+        plan, compiled._native = compiled._native, False  # the same call through the tasklets
+        want = compiled(**dict(zip(module.sdfg.arg_names, args)))
+        compiled._native = plan
+        for g, w in zip(got if isinstance(got, tuple) else (got, ), want if isinstance(want, tuple) else (want, )):
+            assert g.data_ptr() != w.data_ptr() and torch.equal(g, w)
+    assert L.get_context(0).device_status() == 0
+
+
+def test_plan_leaves_other_arguments_to_the_general_path():
+    module = DaceModule(LeNet(), dummy_inputs=(torch.rand(2, 1, 32, 32), ))
+    x = torch.rand(2, 1, 32, 64)
+    strided, dense = x.cuda()[..., ::2], x[..., ::2].contiguous()
+    y = module(dense.cuda())
+    assert torch.equal(module(strided), y)
+    assert torch.equal(module(dense).cpu(), y.cpu())
+    with pytest.raises(ValueError):
+        module(torch.rand(3, 1, 32, 32, device="cuda"))
+    with pytest.raises(ValueError):
+        module(dense.cuda().half())
+
+
+def test_plan_follows_a_replaced_constant():
+    net = nn.Linear(8, 8, bias=False)
+    module = DaceModule(net, dummy_inputs=(torch.rand(4, 8), ))
+    x = torch.rand(4, 8, device="cuda")
+    y = module(x)
+    name = next(n for n, t in module.sdfg.constants.items() if t.numel() == 64)
+    module.sdfg.constants[name] = module.sdfg.constants[name] * 2.0
+    assert torch.equal(module(x), y * 2.0)
