@@ -36,7 +36,9 @@ int fail(int code, const char* fmt, ...) {
 }
 
 int gemm_f16(const b200ml_ctx* ctx, const b200ml_gemm_params* p, cudaStream_t stream);
-int gemm_f32(const b200ml_ctx* ctx, const b200ml_gemm_params* p, cudaStream_t stream);
+int gemm_f32(const b200ml_ctx* ctx, const b200ml_gemm_params* p, const void* packed, cudaStream_t stream);
+int64_t gemm_prepack_bytes(const b200ml_gemm_params* p);
+int gemm_prepack(const b200ml_ctx* ctx, const b200ml_gemm_params* p, void* packed, cudaStream_t stream);
 int gemm_f16_layernorm(const b200ml_ctx* ctx, const b200ml_gemm_params* p, cudaStream_t stream);
 int softmax(int dtype, const void* x, const void* mask, void* y, int64_t rows, int64_t cols, int64_t mask_row_div,
             float scale, int is_log, cudaStream_t s);
@@ -209,7 +211,7 @@ int b200ml_ctx_device_status(b200ml_ctx* ctx, int32_t* status) {
 
 int64_t b200ml_ctx_workspace_bytes(const b200ml_ctx* ctx) { return ctx ? ctx->workspace_bytes : 0; }
 
-int b200ml_gemm(b200ml_ctx* ctx, const b200ml_gemm_params* p, b200ml_stream stream) {
+int b200ml_gemm_packed(b200ml_ctx* ctx, const b200ml_gemm_params* p, const void* packed_b, b200ml_stream stream) {
     CTX_CHECK(ctx);
     B200ML_REQUIRE(p != nullptr, "gemm: null parameter block");
     B200ML_REQUIRE(dtype_ok(p->dtype), "gemm: unknown dtype %d", p->dtype);
@@ -232,7 +234,24 @@ int b200ml_gemm(b200ml_ctx* ctx, const b200ml_gemm_params* p, b200ml_stream stre
         if (p->dtype != B200ML_F16) return fail(B200ML_ERR_UNSUPPORTED, "gemm + layernorm: fp16 only");
         return gemm_f16_layernorm(ctx, p, s);
     }
-    return p->dtype == B200ML_F16 ? gemm_f16(ctx, p, s) : gemm_f32(ctx, p, s);
+    return p->dtype == B200ML_F16 ? gemm_f16(ctx, p, s) : gemm_f32(ctx, p, packed_b, s);
+}
+
+int b200ml_gemm(b200ml_ctx* ctx, const b200ml_gemm_params* p, b200ml_stream stream) { return b200ml_gemm_packed(ctx, p, nullptr, stream); }
+
+int64_t b200ml_gemm_prepack_bytes(b200ml_ctx* ctx, const b200ml_gemm_params* p) {
+    if (ctx == nullptr || p == nullptr) return 0;
+    return gemm_prepack_bytes(p);
+}
+
+int b200ml_gemm_prepack(b200ml_ctx* ctx, const b200ml_gemm_params* p, void* packed, b200ml_stream stream) {
+    CTX_CHECK(ctx);
+    B200ML_REQUIRE(p != nullptr && packed != nullptr, "gemm_prepack: null argument");
+    B200ML_REQUIRE(gemm_prepack_bytes(p) > 0, "gemm_prepack: this product takes no packed operand");
+    B200ML_REQUIRE(p->b && p->ldb >= (p->b_layout ? p->k : p->n) && p->k < (1ll << 31), "gemm_prepack: bad B");
+    B200ML_REQUIRE(aligned16(packed), "gemm_prepack: the packed copy must be 16-byte aligned");
+    DeviceGuard guard(ctx->device);
+    return gemm_prepack(ctx, p, packed, static_cast<cudaStream_t>(stream));
 }
 
 int b200ml_softmax(b200ml_ctx* ctx, int32_t dtype, const void* x, const void* mask, void* y, int64_t rows,

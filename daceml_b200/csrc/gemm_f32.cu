@@ -1,0 +1,792 @@
+// fp32 GEMM on the tensor cores with fp32-grade accuracy ("3 x TF32"), and the GEMMs of either type that the fp16
+// tensor-core kernels cannot address (unaligned rows, transposed A, a handful of rows):
+//     C = act(alpha * A.B + bias) + residual,   A [M, K] or [K, M], B [K, N] or [N, K], two batch loops, any strides.
+//
+// A single TF32 product keeps 11 significant bits of each operand (relative error ~5e-4, outside the 1e-4 the fp32
+// configurations allow).  Each operand is therefore split into hi = the value rounded to TF32 and lo = value - hi (exact in
+// fp32), and the tensor core accumulates  A_lo.B_hi + A_hi.B_lo + A_hi.B_hi  (the dropped A_lo.B_lo term is ~2^-22
+// relative) in fp32 TMEM.  The accumulator add truncates, and that error grows with the number of accumulation steps;
+// the k-blocks are dealt round-robin to four accumulators, which the epilogue adds with round-to-nearest.  fp16 operands
+// are exact in TF32: one product, no lo parts.
+//
+// gemm_f32_kernel: one 128 x BN tile per CTA (or per cluster: K split over 2, 4 or 8 CTAs).  Eight producer warps in two
+// groups that take the k-blocks in turn load the operands with ordinary (16-byte where the rows allow, coalesced) loads
+// one block ahead, split them in registers and write the swizzled operand tiles; one thread issues tcgen05.mma
+// kind::tf32.  So A needs no pass of its own over memory, no workspace and no alignment.  B goes the same way, or - when
+// many row tiles would repeat its split - comes from a copy that was split beforehand, already in the operand tiles'
+// order (f32_pack_kernel: once for a constant weight, once per call otherwise), by plain bulk copies.  Products of many
+// tiles in both directions have A packed by the same launch: then the loads, the split and half of the shared-memory
+// stores leave the kernel (4096 x 768 x 768: 56 us with A split in the kernel, 44 with both packed).
+// The tile's partial sums are parked row-major in shared memory (free by then) and leave as whole rows; with a split K
+// every CTA of the cluster adds up its share of the rows through distributed shared memory, in rank order.
+// What bounds it: shared-memory bandwidth (160 KB written and read per 128 x 128 x 32 block, 1280 cycles against 384 of
+// tensor arithmetic) on large products; latency (launch, first loads, reduction) on small ones.
+//
+// gemm_rows_kernel: up to 32 rows against K-contiguous B: a warp per column and eight rows, lanes along K.  Bound by
+// latency; a 128-row tile would be nearly empty.
+#include "gemm_common.cuh"
+#include "conv_tc.cuh"
+
+namespace b200ml {
+
+namespace {
+
+constexpr int FM = 128, FK = 32;  // 32 fp32 = one 128-byte line of the operand tiles
+constexpr int F_NACC = 4;
+constexpr int F_THREADS = 320;  // warp 0: MMA; warps 1-8: producers, then epilogue; warp 9: copies of a packed B
+constexpr int F_PACK_ROWS = 32; // packed B: rows are padded to a multiple of this
+
+template <typename T, int BN>
+struct F32Smem {
+    static constexpr int PARTS = sizeof(T) == 4 ? 2 : 1;  // hi and lo; fp16 values have no lo part
+    static constexpr int A_BYTES = FM * FK * 4, B_BYTES = BN * FK * 4;
+    static constexpr int STAGE_BYTES = PARTS * (A_BYTES + B_BYTES);
+    static constexpr int STAGES = BN == 128 ? 3 : 4;
+    static constexpr int PART_LD = BN + 4;  // floats between rows of the parked tile: 16-byte rows, no bank conflicts
+    static constexpr int TOTAL = STAGES * STAGE_BYTES + 256 + 1024;
+    static_assert(FM * PART_LD * 4 <= STAGES * STAGE_BYTES, "the parked tile lies over the pipeline stages");
+};
+
+template <typename T>
+struct F32Operand {
+    const T* p;
+    int64_t ld, so, si;
+    int32_t rows;  // M or N
+    int32_t mn;    // 0: K contiguous; 1: M / N contiguous
+    int32_t vec;   // four consecutive elements may be loaded at once
+};
+
+template <typename T>
+struct F32Args {
+    F32Operand<T> a, b;
+    const float* packed_a;  // operands split and tiled beforehand (f32_pack_kernel), or null
+    const float* packed_b;
+    int32_t packed_a_rows, packed_b_rows;  // their padded row counts
+    int32_t m, n, k, tiles_m, tiles_n, batch_inner, split;
+    int32_t b_constant;
+    int32_t c_vec, r_vec, bias_vec;
+    EpilogueParams ep;
+    int64_t ldc, c_so, c_si, ldr, r_so, r_si;
+    T* c;
+    const T* bias;
+    const T* residual;
+    int32_t* status;
+};
+
+__device__ __forceinline__ float to_f(float v) { return v; }
+__device__ __forceinline__ float to_f(__half v) { return __half2float(v); }
+
+// Up to four consecutive elements; those from `valid` on read as zero.
+__device__ __forceinline__ float4 load4(const float* p, bool vec, int valid) {
+    if (vec && valid >= 4) return __ldg(reinterpret_cast<const float4*>(p));
+    return make_float4(valid > 0 ? __ldg(p) : 0.0f, valid > 1 ? __ldg(p + 1) : 0.0f, valid > 2 ? __ldg(p + 2) : 0.0f, valid > 3 ? __ldg(p + 3) : 0.0f);
+}
+__device__ __forceinline__ float4 load4(const __half* p, bool vec, int valid) {
+    if (vec && valid >= 4) {
+        const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
+        const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&q.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
+        return make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+    return make_float4(valid > 0 ? to_f(p[0]) : 0.0f, valid > 1 ? to_f(p[1]) : 0.0f, valid > 2 ? to_f(p[2]) : 0.0f, valid > 3 ? to_f(p[3]) : 0.0f);
+}
+__device__ __forceinline__ void store4(float* p, bool vec, int valid, const float (&v)[4]) {
+    if (vec && valid >= 4) {
+        *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j < valid) p[j] = v[j];
+    }
+}
+__device__ __forceinline__ void store4(__half* p, bool vec, int valid, const float (&v)[4]) {
+    if (vec && valid >= 4) {
+        uint2 q;
+        *reinterpret_cast<__half2*>(&q.x) = __floats2half2_rn(v[0], v[1]);
+        *reinterpret_cast<__half2*>(&q.y) = __floats2half2_rn(v[2], v[3]);
+        *reinterpret_cast<uint2*>(p) = q;
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j < valid) p[j] = __float2half_rn(v[j]);
+    }
+}
+
+// hi = x rounded to nearest-even at 10 mantissa bits (TF32), lo = x - hi; infinities and NaNs stay in hi.
+__device__ __forceinline__ void split_rn(float x, float& hi, float& lo) {
+    const uint32_t b = __float_as_uint(x);
+    const bool finite = (b & 0x7f800000u) != 0x7f800000u;
+    hi = __uint_as_float(finite ? ((b + 0xfffu + ((b >> 13) & 1u)) & 0xffffe000u) : b);
+    lo = finite ? x - hi : 0.0f;
+}
+
+__device__ __forceinline__ void split4(const float4& v, float4& hi, float4& lo) {
+    split_rn(v.x, hi.x, lo.x), split_rn(v.y, hi.y, lo.y), split_rn(v.z, hi.z, lo.z), split_rn(v.w, hi.w, lo.w);
+}
+
+// A 16-byte unit of an operand tile of ROWS rows x 32 k: where it comes from and where it goes.
+//   K contiguous: eight lanes cover a row's 128 bytes; 128-byte swizzle (16-byte chunk ^ row mod 8).
+//   M / N contiguous: a warp covers one k of ROWS columns; per 32 columns a block of 32 lines (one per k) of 128 bytes, the
+//   128-byte swizzle with 32-byte atoms (32-byte chunk ^ k mod 4).
+template <int ROWS, typename T>
+__device__ __forceinline__ float4 operand_load(const F32Operand<T>& o, const T* base, int r0, int k0, int k_end, int u) {
+    if (!o.mn) {
+        const int row = r0 + (u >> 3), k = k0 + (u & 7) * 4;
+        if (row >= o.rows || k >= k_end) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        return load4(base + static_cast<int64_t>(row) * o.ld + k, o.vec, k_end - k);
+    }
+    constexpr int UNITS = ROWS / 4;  // per k
+    const int k = k0 + u / UNITS, row = r0 + (u % UNITS) * 4;
+    if (row >= o.rows || k >= k_end) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    return load4(base + static_cast<int64_t>(k) * o.ld + row, o.vec, o.rows - row);
+}
+template <int ROWS>
+__device__ __forceinline__ uint32_t operand_offset(bool mn, int u) {
+    if (!mn) {
+        const int row = u >> 3, c = u & 7;
+        return row * 128 + ((c ^ (row & 7)) << 4);
+    }
+    constexpr int UNITS = ROWS / 4;
+    const int k = u / UNITS, c = u % UNITS;
+    return (c >> 3) * 4096 + k * 128 + ((((c & 7) >> 1) ^ (k & 3)) << 5) + (c & 1) * 16;
+}
+
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(ptx::smem_u32(bar))
+                 : "memory");
+}
+
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t local_addr, uint32_t rank) {
+    uint32_t raddr;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(raddr) : "r"(local_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(raddr) : "memory");
+    return v;
+}
+
+// alpha, bias, activation, residual of four columns of one row, and their store.
+template <typename T>
+__device__ __forceinline__ void finish4(const F32Args<T>& g, const float4& acc, T* c, const T* res, int row, int col) {
+    const int valid = g.n - col;
+    float v[4] = {g.ep.alpha * acc.x, g.ep.alpha * acc.y, g.ep.alpha * acc.z, g.ep.alpha * acc.w};
+    if ((g.ep.flags & B200ML_EPI_BIAS) && g.bias) {
+        const float4 b = load4(g.bias + col, g.bias_vec, valid);
+        v[0] = fmaf(g.ep.bias_scale, b.x, v[0]), v[1] = fmaf(g.ep.bias_scale, b.y, v[1]);
+        v[2] = fmaf(g.ep.bias_scale, b.z, v[2]), v[3] = fmaf(g.ep.bias_scale, b.w, v[3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = apply_act(v[j], g.ep.flags);
+    if ((g.ep.flags & B200ML_EPI_RESIDUAL) && res) {
+        const float4 q = load4(res + static_cast<int64_t>(row) * g.ldr + col, g.r_vec, valid);
+        v[0] = fmaf(g.ep.residual_scale, q.x, v[0]), v[1] = fmaf(g.ep.residual_scale, q.y, v[1]);
+        v[2] = fmaf(g.ep.residual_scale, q.z, v[2]), v[3] = fmaf(g.ep.residual_scale, q.w, v[3]);
+    }
+    store4(c + static_cast<int64_t>(row) * g.ldc + col, g.c_vec, valid, v);
+}
+
+template <typename T, int BN, bool PACKED_A, bool PACKED_B>
+__global__ void __launch_bounds__(F_THREADS, 1) gemm_f32_kernel(const F32Args<T> g) {
+    using S = F32Smem<T, BN>;
+    constexpr int STAGES = S::STAGES, PARTS = S::PARTS;
+    constexpr uint32_t TMEM_COLS = F_NACC * BN;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * S::STAGE_BYTES);
+    uint64_t* empty_bar = full_bar + STAGES;
+    uint64_t* acc_bar = empty_bar + STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
+
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = g.split > 1 ? static_cast<int>(ptx::cluster_ctarank()) : 0;
+    const int tile = blockIdx.x / g.split;
+    const int m0 = (tile % g.tiles_m) * FM;
+    const int nt = (tile / g.tiles_m) % g.tiles_n, n0 = nt * BN;
+    const int batch = tile / (g.tiles_m * g.tiles_n);
+    const int bi = batch % g.batch_inner, bo = batch / g.batch_inner;
+    const int num_kb = (g.k + FK - 1) / FK;
+    const int kb_per = (num_kb + g.split - 1) / g.split;
+    const int kb_begin = rank * kb_per < num_kb ? rank * kb_per : num_kb;
+    const int nk = (kb_begin + kb_per < num_kb ? kb_begin + kb_per : num_kb) - kb_begin;  // this CTA's share of K, may be 0
+
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int s = 0; s < STAGES; ++s) {
+                // the four warps of a producer group, and the copies of packed operands
+                ptx::mbar_init(&full_bar[s], (PACKED_A ? 0 : 4) + (PACKED_A || PACKED_B ? 1 : 0));
+                ptx::mbar_init(&empty_bar[s], 1);
+            }
+            ptx::mbar_init(acc_bar, 1);
+            ptx::fence_mbar_init();
+        }
+        __syncwarp();
+        ptx::tmem_alloc(tmem_slot, TMEM_COLS);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        // ------------------------------ MMA issuer ------------------------------
+        if (ptx::elect_one()) {
+            const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(PACKED_A ? 0 : g.a.mn) << 15) |
+                                   (static_cast<uint32_t>(PACKED_B ? 0 : g.b.mn) << 16) | ((BN >> 3) << 17) | ((FM >> 4) << 24);
+            bool ok = true;
+            int stage = 0;
+            uint32_t phase = 0;
+            for (int i = 0; i < nk; ++i) {
+                if (!ptx::mbar_wait(&full_bar[stage], phase)) {
+                    atomicExch(g.status, DEV_TIMEOUT_MMA);
+                    ok = false;
+                    break;
+                }
+                ptx::tc_fence_after();
+                const uint32_t d_tmem = tmem_base + (i % F_NACC) * BN;
+                const uint32_t ah = ptx::smem_u32(smem + stage * S::STAGE_BYTES), al = ah + S::A_BYTES;
+                const uint32_t bh = ah + PARTS * S::A_BYTES, bl = bh + S::B_BYTES;
+                const bool a_mn = !PACKED_A && g.a.mn != 0, b_mn = !PACKED_B && g.b.mn != 0;
+#pragma unroll
+                for (int kk = 0; kk < FK / 8; ++kk) {
+                    // K contiguous: 32 bytes along the 128-byte line per step; M / N contiguous: 8 lines (two 4-line groups 512
+                    // bytes apart) per step, blocks of 32 columns 4 KB apart
+                    auto desc = [&](uint32_t addr, bool mn) {
+                        return mn ? convtc::make_smem_desc_sw128_base32(addr + kk * 1024, 4096, 512) : ptx::make_smem_desc_sw128(addr + kk * 32, 16, 1024);
+                    };
+                    const uint32_t first = (i >= F_NACC || kk != 0) ? 1u : 0u;
+                    const uint64_t d_ah = desc(ah, a_mn), d_bh = desc(bh, b_mn);
+                    if constexpr (PARTS == 2) {  // the two small terms first, the large one last
+                        convtc::pw_mma(d_tmem, desc(al, a_mn), d_bh, idesc, first);
+                        convtc::pw_mma(d_tmem, d_ah, desc(bl, b_mn), idesc, 1u);
+                        convtc::pw_mma(d_tmem, d_ah, d_bh, idesc, 1u);
+                    } else {
+                        convtc::pw_mma(d_tmem, d_ah, d_bh, idesc, first);
+                    }
+                }
+                ptx::mma_commit(&empty_bar[stage]);
+                if (++stage == STAGES) stage = 0, phase ^= 1;
+            }
+            if (ok && nk > 0) ptx::mma_commit(acc_bar);
+        }
+        __syncwarp();
+    } else if (warp == 9) {
+        // ------------------------------ packed operands: two bulk copies each per k-block ------------------------------
+        if ((PACKED_A || PACKED_B) && ptx::elect_one()) {
+            if (PACKED_A || !g.b_constant) pdl_wait();
+            int stage = 0;
+            uint32_t phase = 0;
+            const int rows_a = PACKED_A ? (g.packed_a_rows - m0 < FM ? g.packed_a_rows - m0 : FM) : 0;
+            const int rows_b = PACKED_B ? (g.packed_b_rows - n0 < BN ? g.packed_b_rows - n0 : BN) : 0;
+            for (int i = 0; i < nk; ++i) {
+                if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
+                    atomicExch(g.status, DEV_TIMEOUT_PRODUCER);
+                    break;
+                }
+                const uint32_t dst = ptx::smem_u32(smem + stage * S::STAGE_BYTES);
+                ptx::mbar_expect_tx(&full_bar[stage], 2 * 128 * (rows_a + rows_b));
+                if (PACKED_A) {
+                    const float* src = g.packed_a + (static_cast<int64_t>(kb_begin + i) * 2 * g.packed_a_rows + m0) * FK;
+                    bulk_copy(dst, src, rows_a * 128, &full_bar[stage]);
+                    bulk_copy(dst + S::A_BYTES, src + static_cast<int64_t>(g.packed_a_rows) * FK, rows_a * 128, &full_bar[stage]);
+                }
+                if (PACKED_B) {
+                    const float* src = g.packed_b + (static_cast<int64_t>(kb_begin + i) * 2 * g.packed_b_rows + n0) * FK;
+                    bulk_copy(dst + PARTS * S::A_BYTES, src, rows_b * 128, &full_bar[stage]);
+                    bulk_copy(dst + PARTS * S::A_BYTES + S::B_BYTES, src + static_cast<int64_t>(g.packed_b_rows) * FK, rows_b * 128, &full_bar[stage]);
+                }
+                if (++stage == STAGES) stage = 0, phase ^= 1;
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------ producers ------------------------------
+        pdl_wait();
+        const int group = (warp - 1) >> 2, t = ((warp - 1) & 3) * 32 + lane;
+        constexpr int UA = FM * 8 / 128, UB = BN * 8 / 128;  // units per thread
+        const T* a_base = g.a.p + bo * g.a.so + bi * g.a.si;
+        const T* b_base = g.b.p + bo * g.b.so + bi * g.b.si;
+        float4 ra[UA], rb[UB];
+        auto load = [&](int i) {
+            const int k0 = (kb_begin + i) * FK;
+#pragma unroll
+            for (int u = 0; u < UA; ++u) ra[u] = operand_load<FM>(g.a, a_base, m0, k0, g.k, u * 128 + t);
+            if (!PACKED_B) {
+#pragma unroll
+                for (int u = 0; u < UB; ++u) rb[u] = operand_load<BN>(g.b, b_base, n0, k0, g.k, u * 128 + t);
+            }
+        };
+        if (!PACKED_A && group < nk) load(group);
+        for (int i = group; !PACKED_A && i < nk; i += 2) {
+            const int stage = i % STAGES;
+            if (!ptx::mbar_wait(&empty_bar[stage], ((i / STAGES) & 1) ^ 1)) {
+                if (lane == 0) atomicExch(g.status, DEV_TIMEOUT_PRODUCER);
+                break;
+            }
+            const uint32_t sa = ptx::smem_u32(smem + stage * S::STAGE_BYTES), sb = sa + PARTS * S::A_BYTES;
+#pragma unroll
+            for (int u = 0; u < UA; ++u) {
+                const uint32_t at = sa + operand_offset<FM>(g.a.mn != 0, u * 128 + t);
+                if constexpr (PARTS == 2) {
+                    float4 hi, lo;
+                    split4(ra[u], hi, lo);
+                    convtc::st_shared_v4(at, hi);
+                    convtc::st_shared_v4(at + S::A_BYTES, lo);
+                } else {
+                    convtc::st_shared_v4(at, ra[u]);
+                }
+            }
+            if (!PACKED_B) {
+#pragma unroll
+                for (int u = 0; u < UB; ++u) {
+                    const uint32_t at = sb + operand_offset<BN>(g.b.mn != 0, u * 128 + t);
+                    if constexpr (PARTS == 2) {
+                        float4 hi, lo;
+                        split4(rb[u], hi, lo);
+                        convtc::st_shared_v4(at, hi);
+                        convtc::st_shared_v4(at + S::B_BYTES, lo);
+                    } else {
+                        convtc::st_shared_v4(at, rb[u]);
+                    }
+                }
+            }
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&full_bar[stage]);
+            if (i + 2 < nk) load(i + 2);
+        }
+        __syncwarp();
+        // ------------------------------ accumulators -> parked tile: 32 rows x BN / 2 columns per warp ------------------------------
+        float* partial = reinterpret_cast<float*>(smem);
+        const int quarter = warp & 3, half = (warp - 1) >> 2;
+        const int row = quarter * 32 + lane;
+        const int nacc = nk < F_NACC ? nk : F_NACC;
+        bool ok = true;
+        if (nk > 0 && !ptx::mbar_wait(acc_bar, 0)) {
+            if (lane == 0) atomicExch(g.status, DEV_TIMEOUT_EPILOGUE);
+            ok = false;
+        }
+        __syncwarp();
+        ptx::tc_fence_after();
+        const uint32_t t_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+#pragma unroll 1
+        for (int c = half * (BN / 2); ok && c < (half + 1) * (BN / 2); c += 16) {
+            if (n0 + c >= g.n) break;  // warp-uniform
+            float v[16];
+            if (nk == 0) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = 0.0f;
+            } else {
+                uint32_t r[F_NACC][16];
+#pragma unroll
+                for (int a = 0; a < F_NACC; ++a)
+                    if (a < nacc) ptx::tmem_ld_32x32b_x16(t_base + a * BN + c, r[a]);
+                ptx::tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[0][j]);
+#pragma unroll
+                for (int a = 1; a < F_NACC; ++a)
+                    if (a < nacc) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[a][j]);
+                    }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<float4*>(partial + row * S::PART_LD + c + 4 * j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        }
+        ptx::tc_fence_before();
+    }
+
+    if (g.split > 1) ptx::cluster_sync_acq_rel();
+    else __syncthreads();
+    if (warp >= 1 && warp <= 8) {
+        // ------------------------------ whole rows out; with a split K this CTA's share of them ------------------------------
+        constexpr int C4 = BN / 4, ROWS_PER_PASS = 256 / C4;
+        const int t = threadIdx.x - 32;
+        const int share = FM / g.split;
+        const int col = n0 + (t % C4) * 4;
+        T* c = g.c + bo * g.c_so + bi * g.c_si;
+        const T* res = g.residual ? g.residual + bo * g.r_so + bi * g.r_si : nullptr;
+        const uint32_t part_addr = ptx::smem_u32(smem);
+        if (col < g.n) {
+            for (int r = t / C4; r < share; r += ROWS_PER_PASS) {
+                const int rt = rank * share + r, row = m0 + rt;
+                if (row >= g.m) break;
+                const uint32_t at = part_addr + (rt * S::PART_LD + (t % C4) * 4) * 4;
+                float4 v;
+                if (g.split == 1) {
+                    v = convtc::ld_shared_v4(at);
+                } else {
+                    v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    for (int q = 0; q < g.split; ++q) {  // rank order: the same sum on every run
+                        const float4 w = ld_cluster_v4(at, q);
+                        v.x += w.x, v.y += w.y, v.z += w.z, v.w += w.w;
+                    }
+                }
+                finish4(g, v, c, res, row, col);
+            }
+        }
+    }
+    if (g.split > 1) ptx::cluster_sync_acq_rel();  // no CTA leaves while a peer may still read its partial tile
+    ptx::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        ptx::tc_fence_after();
+        if (*reinterpret_cast<volatile int32_t*>(g.status) != DEV_OK) {
+            for (int i = 0; i < 200; ++i) __nanosleep(1000);  // a wait gave up: let copies and MMAs in flight land
+        }
+        ptx::tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+}
+
+// An operand split into hi and lo and laid out as the operand tiles: [k-block][hi | lo][row (padded)][32 k], 128-byte swizzle
+// inside each group of eight rows; rows and k past the end are zero.  A thread makes one 16-byte unit of each part; the
+// first `first_blocks` blocks take the first operand, the others the second.
+struct PackJob {
+    F32Operand<float> o;
+    float* out;
+    int32_t rows_padded;
+    int64_t units;
+};
+
+__global__ void __launch_bounds__(256) f32_pack_kernel(const PackJob ja, const PackJob jb, int32_t k, unsigned first_blocks) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const bool first = blockIdx.x < first_blocks;
+    const PackJob& j = first ? ja : jb;
+    const int64_t block = first ? blockIdx.x : blockIdx.x - first_blocks, blocks = first ? first_blocks : gridDim.x - first_blocks;
+    const F32Operand<float>& b = j.o;
+    for (int64_t i = block * blockDim.x + threadIdx.x; i < j.units; i += blocks * blockDim.x) {
+        int row, c;
+        int64_t kb;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (!b.mn) {  // consecutive threads along k
+            c = static_cast<int>(i & 7);
+            const int64_t rest = i >> 3;
+            row = static_cast<int>(rest % j.rows_padded), kb = rest / j.rows_padded;
+            const int kk = static_cast<int>(kb) * FK + c * 4;
+            if (row < b.rows && kk < k) v = load4(b.p + static_cast<int64_t>(row) * b.ld + kk, b.vec, k - kk);
+        } else {  // consecutive threads along the rows
+            row = static_cast<int>(i % j.rows_padded);
+            const int64_t rest = i / j.rows_padded;
+            c = static_cast<int>(rest & 7), kb = rest >> 3;
+            const int kk = static_cast<int>(kb) * FK + c * 4;
+            if (row < b.rows) {
+                const float* p = b.p + static_cast<int64_t>(kk) * b.ld + row;
+                v.x = kk < k ? __ldg(p) : 0.0f, v.y = kk + 1 < k ? __ldg(p + b.ld) : 0.0f;
+                v.z = kk + 2 < k ? __ldg(p + 2 * b.ld) : 0.0f, v.w = kk + 3 < k ? __ldg(p + 3 * b.ld) : 0.0f;
+            }
+        }
+        float4 hi, lo;
+        split4(v, hi, lo);
+        float* dst = j.out + (kb * 2 * j.rows_padded + row) * FK + ((c ^ (row & 7)) << 2);
+        *reinterpret_cast<float4*>(dst) = hi;
+        *reinterpret_cast<float4*>(dst + static_cast<int64_t>(j.rows_padded) * FK) = lo;
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// A few rows: a warp per column and up to MB rows, lanes along K.
+// ---------------------------------------------------------------------------------------------
+template <typename T>
+struct RowsArgs {
+    const T* a;
+    const T* b;
+    const T* bias;
+    const T* residual;
+    T* c;
+    int64_t lda, ldb, ldc, ldr, a_so, a_si, b_so, b_si, c_so, c_si, r_so, r_si;
+    int32_t m, n, k, batch_inner, vec, b_constant;
+    EpilogueParams ep;
+};
+
+template <typename T>
+struct Packet;
+template <>
+struct Packet<float> {
+    static constexpr int N = 4;
+    float v[4];
+    __device__ __forceinline__ void load(const float* p) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+    }
+};
+template <>
+struct Packet<__half> {
+    static constexpr int N = 8;
+    float v[8];
+    __device__ __forceinline__ void load(const __half* p) { unpack8(__ldg(reinterpret_cast<const uint4*>(p)), v); }
+};
+
+constexpr int ROWS_WARPS = 4;
+
+template <typename T, int MB>
+__global__ void __launch_bounds__(32 * ROWS_WARPS) gemm_rows_kernel(const RowsArgs<T> g) {
+    using P = Packet<T>;
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31;
+    const int n = blockIdx.x * ROWS_WARPS + (threadIdx.x >> 5);
+    const int m0 = blockIdx.y * MB;
+    const int bi = blockIdx.z % g.batch_inner, bo = blockIdx.z / g.batch_inner;
+    if (n >= g.n) return;
+    const T* b = g.b + bo * g.b_so + bi * g.b_si + static_cast<int64_t>(n) * g.ldb;
+    const T* a = g.a + bo * g.a_so + bi * g.a_si;
+    float acc[MB];
+#pragma unroll
+    for (int i = 0; i < MB; ++i) acc[i] = 0.0f;
+    const T* ar[MB];
+#pragma unroll
+    for (int i = 0; i < MB; ++i) ar[i] = a + static_cast<int64_t>(m0 + i < g.m ? m0 + i : g.m - 1) * g.lda;
+    if (g.vec) {
+        // A constant weight does not depend on the kernel in front: its first packets are requested before the wait.
+        constexpr int PRE = 3;
+        P pre[PRE];
+        const int first = lane * P::N;
+        if (g.b_constant) {
+#pragma unroll
+            for (int u = 0; u < PRE; ++u)
+                if (first + u * 32 * P::N < g.k) pre[u].load(b + first + u * 32 * P::N);
+        }
+        pdl_wait();
+        if (!g.b_constant) {
+#pragma unroll
+            for (int u = 0; u < PRE; ++u)
+                if (first + u * 32 * P::N < g.k) pre[u].load(b + first + u * 32 * P::N);
+        }
+        auto add = [&](const P& w, int k) {
+#pragma unroll
+            for (int i = 0; i < MB; ++i) {
+                P x;
+                x.load(ar[i] + k);
+#pragma unroll
+                for (int j = 0; j < P::N; ++j) acc[i] = fmaf(x.v[j], w.v[j], acc[i]);
+            }
+        };
+#pragma unroll
+        for (int u = 0; u < PRE; ++u)
+            if (first + u * 32 * P::N < g.k) add(pre[u], first + u * 32 * P::N);
+#pragma unroll 4
+        for (int k = first + PRE * 32 * P::N; k < g.k; k += 32 * P::N) {
+            P w;
+            w.load(b + k);
+            add(w, k);
+        }
+    } else {
+        pdl_wait();
+#pragma unroll 4
+        for (int k = lane; k < g.k; k += 32) {
+            const float w = to_f(b[k]);
+#pragma unroll
+            for (int i = 0; i < MB; ++i) acc[i] = fmaf(to_f(ar[i][k]), w, acc[i]);
+        }
+    }
+    float mine = 0.0f;
+#pragma unroll
+    for (int i = 0; i < MB; ++i) {
+        float v = acc[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == i) mine = v;
+    }
+    const int row = m0 + lane;
+    if (lane < MB && row < g.m) {
+        float v = g.ep.alpha * mine;
+        if ((g.ep.flags & B200ML_EPI_BIAS) && g.bias) v = fmaf(g.ep.bias_scale, to_f(g.bias[n]), v);
+        v = apply_act(v, g.ep.flags);
+        if ((g.ep.flags & B200ML_EPI_RESIDUAL) && g.residual)
+            v = fmaf(g.ep.residual_scale, to_f(g.residual[bo * g.r_so + bi * g.r_si + static_cast<int64_t>(row) * g.ldr + n]), v);
+        T* c = g.c + bo * g.c_so + bi * g.c_si + static_cast<int64_t>(row) * g.ldc + n;
+        if constexpr (sizeof(T) == 4) *c = v;
+        else *c = __float2half_rn(v);
+    }
+}
+
+template <typename T>
+int launch_rows(const b200ml_gemm_params* p, cudaStream_t stream) {
+    RowsArgs<T> g{};
+    g.a = static_cast<const T*>(p->a), g.b = static_cast<const T*>(p->b), g.bias = static_cast<const T*>(p->bias);
+    g.residual = static_cast<const T*>(p->residual), g.c = static_cast<T*>(p->c);
+    g.lda = p->lda, g.ldb = p->ldb, g.ldc = p->ldc, g.ldr = p->ldr;
+    g.a_so = p->a_stride_outer, g.a_si = p->a_stride_inner, g.b_so = p->b_stride_outer, g.b_si = p->b_stride_inner;
+    g.c_so = p->c_stride_outer, g.c_si = p->c_stride_inner, g.r_so = p->r_stride_outer, g.r_si = p->r_stride_inner;
+    g.m = (int32_t)p->m, g.n = (int32_t)p->n, g.k = (int32_t)p->k, g.batch_inner = (int32_t)p->batch_inner;
+    constexpr int N = Packet<T>::N;
+    g.vec = aligned16(p->a) && aligned16(p->b) && p->k % N == 0 && p->lda % N == 0 && p->ldb % N == 0 && p->a_stride_inner % N == 0 &&
+            p->a_stride_outer % N == 0 && p->b_stride_inner % N == 0 && p->b_stride_outer % N == 0;
+    g.b_constant = (p->flags & B200ML_GEMM_B_CONSTANT) ? 1 : 0;
+    g.ep = EpilogueParams{p->epilogue, p->alpha, p->bias_scale, p->residual_scale};
+    const unsigned batches = (unsigned)(p->batch_outer * p->batch_inner);
+    const unsigned gx = (unsigned)ceil_div(p->n, ROWS_WARPS);
+    const dim3 block(32 * ROWS_WARPS);
+    if (p->m == 1) B200ML_CUDA(launch_pdl(gemm_rows_kernel<T, 1>, dim3(gx, 1, batches), block, 0, stream, g));
+    else if (p->m == 2) B200ML_CUDA(launch_pdl(gemm_rows_kernel<T, 2>, dim3(gx, 1, batches), block, 0, stream, g));
+    else if (p->m <= 4) B200ML_CUDA(launch_pdl(gemm_rows_kernel<T, 4>, dim3(gx, 1, batches), block, 0, stream, g));
+    else B200ML_CUDA(launch_pdl(gemm_rows_kernel<T, 8>, dim3(gx, (unsigned)ceil_div(p->m, 8), batches), block, 0, stream, g));
+    return check_launch("gemm_rows");
+}
+
+// The row kernel repeats B for every eight rows and runs on the FMA pipe: it wins while the 128-row tiles are mostly empty.
+bool rows_applies(const b200ml_gemm_params* p) {
+    return p->a_layout == 0 && p->b_layout == 1 && p->m <= 32 && p->batch_outer * p->batch_inner <= 65535;
+}
+
+template <typename T, int BN, bool PACKED_A, bool PACKED_B>
+int launch_f32(const b200ml_ctx* ctx, F32Args<T>& g, int64_t tiles, int split, cudaStream_t stream) {
+    using S = F32Smem<T, BN>;
+    auto kernel = gemm_f32_kernel<T, BN, PACKED_A, PACKED_B>;
+    static bool configured[64] = {};  // per instantiation and device
+    if (!configured[ctx->device & 63]) {
+        B200ML_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
+        configured[ctx->device & 63] = true;
+    }
+    g.split = split;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * split));
+    cfg.blockDim = dim3(F_THREADS);
+    cfg.dynamicSmemBytes = S::TOTAL;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = split, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    B200ML_CUDA(cudaLaunchKernelEx(&cfg, kernel, g));
+    return check_launch("gemm_f32");
+}
+
+template <typename T>
+F32Operand<T> operand(const void* p, int64_t ld, int64_t so, int64_t si, int64_t rows, bool mn) {
+    F32Operand<T> o{static_cast<const T*>(p), ld, so, si, (int32_t)rows, mn ? 1 : 0, 0};
+    o.vec = (reinterpret_cast<uintptr_t>(p) % (4 * sizeof(T)) == 0 && ld % 4 == 0 && so % 4 == 0 && si % 4 == 0) ? 1 : 0;
+    return o;
+}
+
+int64_t packed_rows(int64_t n) { return ceil_div(n, F_PACK_ROWS) * F_PACK_ROWS; }
+int64_t packed_bytes(int64_t n, int64_t k) { return ceil_div(k, FK) * 2 * packed_rows(n) * FK * 4; }
+
+PackJob pack_job(const F32Operand<float>& o, int64_t k, float* out) {
+    const int64_t rows = packed_rows(o.rows);
+    return PackJob{o, out, (int32_t)rows, ceil_div(k, FK) * rows * 8};
+}
+
+// Packs one or two operands (an operand without units is skipped) in one launch.
+int pack(const b200ml_ctx* ctx, const PackJob& a, const PackJob& b, int64_t k, cudaStream_t stream) {
+    const int64_t cap = (int64_t)ctx->sm_count * 16;
+    const auto blocks = [&](const PackJob& j) { return (unsigned)(ceil_div(j.units, 256) < cap ? ceil_div(j.units, 256) : cap); };
+    B200ML_CUDA(launch_pdl(f32_pack_kernel, dim3(blocks(a) + blocks(b)), dim3(256), 0, stream, a, b, (int32_t)k, blocks(a)));
+    return check_launch("f32_pack");
+}
+
+template <typename T>
+int gemm_f32_impl(const b200ml_ctx* ctx, const b200ml_gemm_params* p, const float* packed_a, const float* packed_b, cudaStream_t stream) {
+    F32Args<T> g{};
+    g.a = operand<T>(p->a, p->lda, p->a_stride_outer, p->a_stride_inner, p->m, p->a_layout == 1);
+    g.b = operand<T>(p->b, p->ldb, p->b_stride_outer, p->b_stride_inner, p->n, p->b_layout == 0);
+    const int64_t batches = p->batch_outer * p->batch_inner;
+    g.packed_a = packed_a, g.packed_b = packed_b;
+    g.packed_a_rows = (int32_t)packed_rows(p->m), g.packed_b_rows = (int32_t)packed_rows(p->n);
+    g.m = (int32_t)p->m, g.n = (int32_t)p->n, g.k = (int32_t)p->k, g.batch_inner = (int32_t)p->batch_inner;
+    g.b_constant = (p->flags & B200ML_GEMM_B_CONSTANT) ? 1 : 0;
+    g.ep = EpilogueParams{p->epilogue, p->alpha, p->bias_scale, p->residual_scale};
+    g.ldc = p->ldc, g.c_so = p->c_stride_outer, g.c_si = p->c_stride_inner;
+    g.ldr = p->ldr, g.r_so = p->r_stride_outer, g.r_si = p->r_stride_inner;
+    g.c = static_cast<T*>(p->c), g.bias = static_cast<const T*>(p->bias), g.residual = static_cast<const T*>(p->residual);
+    g.c_vec = operand<T>(p->c, p->ldc, p->c_stride_outer, p->c_stride_inner, 0, false).vec;
+    g.r_vec = operand<T>(p->residual, p->ldr, p->r_stride_outer, p->r_stride_inner, 0, false).vec;
+    g.bias_vec = reinterpret_cast<uintptr_t>(p->bias) % (4 * sizeof(T)) == 0 ? 1 : 0;
+    g.status = ctx->status_dev;
+    g.tiles_m = (int32_t)ceil_div(p->m, FM);
+    const int num_kb = (int)ceil_div(p->k, FK);
+    // Tile width: narrow outputs get narrow tiles; so do products that would leave most SMs idle even with K split eight ways.
+    int bn = p->n <= 32 ? 32 : (p->n <= 64 ? 64 : 128);
+    if (!packed_a && bn == 128 && g.tiles_m * ceil_div(p->n, 128) * batches * 8 <= ctx->sm_count) bn = 64;
+    g.tiles_n = (int32_t)ceil_div(p->n, bn);
+    const int64_t tiles = (int64_t)g.tiles_m * g.tiles_n * batches;
+    B200ML_REQUIRE(tiles < (1ll << 27), "gemm: too many tiles");
+    // Few output tiles: K is split over a cluster per tile while that adds CTAs and every CTA keeps two k-blocks.
+    int split = 1;
+    while (split < 8 && tiles * split * 2 <= ctx->sm_count && num_kb >= split * 4) split *= 2;
+    if constexpr (sizeof(T) == 4) {
+        if (packed_a) return launch_f32<float, 128, true, true>(ctx, g, tiles, split, stream);  // bn is 128: see pack_a_pays
+        if (packed_b) {
+            switch (bn) {
+                case 32: return launch_f32<float, 32, false, true>(ctx, g, tiles, split, stream);
+                case 64: return launch_f32<float, 64, false, true>(ctx, g, tiles, split, stream);
+                default: return launch_f32<float, 128, false, true>(ctx, g, tiles, split, stream);
+            }
+        }
+    }
+    switch (bn) {
+        case 32: return launch_f32<T, 32, false, false>(ctx, g, tiles, split, stream);
+        case 64: return launch_f32<T, 64, false, false>(ctx, g, tiles, split, stream);
+        default: return launch_f32<T, 128, false, false>(ctx, g, tiles, split, stream);
+    }
+}
+
+// A is packed as well when four or more column tiles would split it again and there is more than a wave of tiles to feed.
+bool pack_a_pays(const b200ml_ctx* ctx, int64_t m, int64_t n) {
+    const int64_t tn = ceil_div(n, 128);
+    return tn >= 4 && ceil_div(m, FM) * tn > ctx->sm_count;
+}
+
+}  // namespace
+
+// Bytes of B in packed form (b200ml_gemm_prepack), 0 where the product does not use one: batched products, and few rows.
+int64_t gemm_prepack_bytes(const b200ml_gemm_params* p) {
+    if (p->dtype != B200ML_F32 || p->batch_outer * p->batch_inner != 1 || p->m < 1 || p->n < 1 || p->k < 1) return 0;
+    if (rows_applies(p) || p->n >= (1ll << 24)) return 0;
+    return packed_bytes(p->n, p->k);
+}
+
+int gemm_prepack(const b200ml_ctx* ctx, const b200ml_gemm_params* p, void* packed, cudaStream_t stream) {
+    const F32Operand<float> b = operand<float>(p->b, p->ldb, 0, 0, p->n, p->b_layout == 0);
+    return pack(ctx, PackJob{}, pack_job(b, p->k, static_cast<float*>(packed)), p->k, stream);
+}
+
+int gemm_f32(const b200ml_ctx* ctx, const b200ml_gemm_params* p, const void* packed, cudaStream_t stream) {
+    if (rows_applies(p)) return launch_rows<float>(p, stream);
+    const float* packed_b = static_cast<const float*>(packed);
+    if (p->batch_outer * p->batch_inner != 1) return gemm_f32_impl<float>(ctx, p, nullptr, nullptr, stream);
+    // B that arrives at run time is packed when at least two row tiles would split it again.
+    const int64_t b_bytes = packed_b ? 0 : packed_bytes(p->n, p->k);
+    const bool pack_b = !packed_b && p->m > FM && p->n >= 32 && p->k >= 64 && p->n < (1ll << 24) && b_bytes <= ctx->workspace_bytes;
+    const bool pack_a = (packed_b || pack_b) && pack_a_pays(ctx, p->m, p->n);
+    if (!pack_b && !pack_a) return gemm_f32_impl<float>(ctx, p, nullptr, packed_b, stream);
+    // the rows of A in pieces whose packed form fits what B leaves of the workspace
+    int64_t rows = p->m;
+    if (pack_a) {
+        const int64_t fit = (ctx->workspace_bytes - (pack_b ? b_bytes : 0)) / packed_bytes(F_PACK_ROWS, p->k) * F_PACK_ROWS / FM * FM;
+        if (fit < FM) return gemm_f32_impl<float>(ctx, p, nullptr, packed_b, stream);
+        const int64_t pieces = ceil_div(p->m, fit);
+        rows = ceil_div(ceil_div(p->m, pieces), FM) * FM;
+    }
+    float* ws_b = static_cast<float*>(ctx->workspace);
+    float* ws_a = ws_b + (pack_b ? b_bytes / 4 : 0);
+    for (int64_t m0 = 0; m0 < p->m; m0 += rows) {
+        b200ml_gemm_params q = *p;
+        q.m = p->m - m0 < rows ? p->m - m0 : rows;
+        q.a = static_cast<const float*>(p->a) + m0 * (p->a_layout ? 1 : p->lda);
+        q.c = static_cast<float*>(p->c) + m0 * p->ldc;
+        if (p->residual) q.residual = static_cast<const float*>(p->residual) + m0 * p->ldr;
+        if (pack_b) q.flags &= ~B200ML_GEMM_B_CONSTANT;  // the workspace is written by the launch just made
+        PackJob ja{}, jb{};
+        if (pack_a) ja = pack_job(operand<float>(q.a, p->lda, 0, 0, q.m, p->a_layout == 1), p->k, ws_a);
+        if (pack_b && m0 == 0) jb = pack_job(operand<float>(p->b, p->ldb, 0, 0, p->n, p->b_layout == 0), p->k, ws_b);
+        int rc = pack(ctx, ja, jb, p->k, stream);
+        if (rc) return rc;
+        rc = gemm_f32_impl<float>(ctx, &q, pack_a ? ws_a : nullptr, pack_b ? ws_b : packed_b, stream);
+        if (rc) return rc;
+    }
+    return B200ML_OK;
+}
+
+// fp16 operands the tensor-core kernels of that type cannot address, and outputs too small for them.
+int gemm_f16_general(const b200ml_ctx* ctx, const b200ml_gemm_params* p, cudaStream_t stream) {
+    if (rows_applies(p)) return launch_rows<__half>(p, stream);
+    return gemm_f32_impl<__half>(ctx, p, nullptr, nullptr, stream);
+}
+
+}  // namespace b200ml

@@ -390,7 +390,7 @@ int launch(const b200ml_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, 
 
 }  // namespace
 
-int gemm_f16_simt(const b200ml_ctx* ctx, const b200ml_gemm_params* p, cudaStream_t stream);
+int gemm_f16_general(const b200ml_ctx* ctx, const b200ml_gemm_params* p, cudaStream_t stream);
 int gemm_f16_pair(const b200ml_ctx* ctx, const b200ml_gemm_params* p, GemmArgs& args, int bn, cudaStream_t stream);
 
 // B200ML_GEMM_PAIR=0 keeps every GEMM on the one-CTA kernel (for A/B comparisons).
@@ -410,11 +410,11 @@ static int pick_bn(int64_t n) { return n > 128 ? 256 : (n > 64 ? 128 : 64); }
 
 int gemm_f16(const b200ml_ctx* ctx, const b200ml_gemm_params* p, cudaStream_t stream) {
     const int64_t batches = p->batch_outer * p->batch_inner;
-    // Operand layouts the tensor-core kernel cannot address go to the FP32-FMA kernel instead.
+    // Operand layouts this kernel cannot address, and outputs of a few rows or values, go to the general kernels.
     const bool a_ok = p->a_layout == 0 && aligned16(p->a) && p->lda % 8 == 0 && p->a_stride_inner % 8 == 0 &&
                       p->a_stride_outer % 8 == 0;
     const bool b_ok = aligned16(p->b) && p->ldb % 8 == 0 && p->b_stride_inner % 8 == 0 && p->b_stride_outer % 8 == 0;
-    if (!a_ok || !b_ok || p->m * p->n * batches < 64 * 64) return gemm_f16_simt(ctx, p, stream);
+    if (!a_ok || !b_ok || p->m * p->n * batches < 64 * 64 || (p->m <= 8 && p->b_layout == 1)) return gemm_f16_general(ctx, p, stream);
 
     const int bn = pick_bn(p->n);
     GemmArgs args{};

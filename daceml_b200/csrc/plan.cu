@@ -24,7 +24,7 @@ enum PlanOp : int32_t {
 };
 // Words of each call: its arguments between the context and the stream, in order.  A structure or an array is stored in
 // the blob itself and its word holds its offset.
-constexpr int kWords[P_COUNT] = {1, 9, 10, 7, 7, 9, 8, 6, 5, 1, 10, 1, 7, 8, 8, 10, 9, 14};
+constexpr int kWords[P_COUNT] = {2, 9, 10, 7, 7, 9, 8, 6, 5, 1, 10, 1, 7, 8, 8, 10, 9, 14};
 
 struct Patch {
     int64_t at;      // byte offset of the pointer in the blob
@@ -63,7 +63,7 @@ using namespace b200ml;
 
 static int plan_call(b200ml_ctx* ctx, int32_t op, const Words& a, b200ml_stream s) {
     switch (op) {
-        case P_GEMM: return b200ml_gemm(ctx, a.at<b200ml_gemm_params>(0), s);
+        case P_GEMM: return b200ml_gemm_packed(ctx, a.at<b200ml_gemm_params>(0), a.p(1), s);
         case P_SOFTMAX:
             return b200ml_softmax(ctx, a.i32(0), a.p(1), a.p(2), a.p(3), a.i64(4), a.i64(5), a.i64(6), a.f(7), a.i32(8), s);
         case P_LAYERNORM:

@@ -34,8 +34,27 @@ def _contig(t, name):
         raise L.B200Error(L.ERR_INVALID, f"{name} must be contiguous")
 
 
-def gemm_raw(ctx, params, stream):
-    L.check(ctx.lib.b200ml_gemm(ctx.handle, ctypes.byref(params), stream))
+def gemm_raw(ctx, params, stream, packed=None):
+    L.check(ctx.lib.b200ml_gemm_packed(ctx.handle, ctypes.byref(params), L.ptr(packed), stream))
+
+
+def gemm_prepack(b, *, n, k, m, b_layout, a_layout=0):
+    """Splits a constant fp32 matrix product operand once (``b200ml_gemm_prepack``): returns the packed tensor to pass on as
+    ``packed``, or None when the product ``[m, k] x b`` takes the operand as it is."""
+    if not b.is_cuda or b.dtype != torch.float32 or not b.is_contiguous():
+        return None
+    ctx = _ctx(b)
+    p = L.GemmParams()
+    p.dtype, p.a_layout, p.b_layout = L.F32, a_layout, b_layout
+    p.m, p.n, p.k, p.batch_outer, p.batch_inner = m, n, k, 1, 1
+    p.lda, p.ldb, p.ldc = (m if a_layout else k), (k if b_layout else n), n
+    p.b = b.data_ptr()
+    nbytes = int(ctx.lib.b200ml_gemm_prepack_bytes(ctx.handle, ctypes.byref(p)))
+    if nbytes <= 0:
+        return None
+    packed = torch.empty(nbytes, dtype=torch.uint8, device=b.device)
+    L.check(ctx.lib.b200ml_gemm_prepack(ctx.handle, ctypes.byref(p), L.ptr(packed), _stream(b)))
+    return packed
 
 
 def gemm(a, b, out, *, b_layout=0, a_layout=0, bias=None, residual=None, act=0, alpha=1.0, bias_scale=1.0,

@@ -34,6 +34,7 @@ EXPORTED_SYMBOLS = [
     "b200ml_where", "b200ml_compare", "b200ml_maxpool2d", "b200ml_wait_probe", "b200ml_strided_copy_parts",
     "b200ml_peer_allgather", "b200ml_ipc_export", "b200ml_ipc_open", "b200ml_ipc_close",
     "b200ml_conv_prepack_bytes", "b200ml_conv_prepack", "b200ml_plan_create", "b200ml_plan_destroy", "b200ml_plan_run",
+    "b200ml_gemm_prepack_bytes", "b200ml_gemm_prepack", "b200ml_gemm_packed",
 ]
 
 
@@ -133,6 +134,10 @@ def load_library(path=None):
         lib.b200ml_last_error.restype = ctypes.c_char_p
         lib.b200ml_launch_count.restype = c_i64
         lib.b200ml_gemm.argtypes = [vp, ctypes.POINTER(GemmParams), vp]
+        lib.b200ml_gemm_packed.argtypes = [vp, ctypes.POINTER(GemmParams), vp, vp]
+        lib.b200ml_gemm_prepack_bytes.argtypes = [vp, ctypes.POINTER(GemmParams)]
+        lib.b200ml_gemm_prepack_bytes.restype = ctypes.c_int64
+        lib.b200ml_gemm_prepack.argtypes = [vp, ctypes.POINTER(GemmParams), vp, vp]
         lib.b200ml_softmax.argtypes = [vp, c_i32, vp, vp, vp, c_i64, c_i64, c_i64, c_f, c_i32, vp]
         lib.b200ml_layernorm.argtypes = [vp, c_i32, vp, vp, vp, vp, vp, vp, c_i64, c_i64, c_f, vp]
         lib.b200ml_reduce.argtypes = [vp, c_i32, c_i32, vp, vp, c_i64, c_i64, c_i64, vp]
@@ -164,7 +169,8 @@ def load_library(path=None):
         lib.b200ml_plan_run.argtypes = [vp, vp, vp, c_i32, vp]
         for name in EXPORTED_SYMBOLS:
             fn = getattr(lib, name)
-            if name not in ("b200ml_last_error", "b200ml_launch_count", "b200ml_ctx_workspace_bytes", "b200ml_conv_prepack_bytes"):
+            if name not in ("b200ml_last_error", "b200ml_launch_count", "b200ml_ctx_workspace_bytes", "b200ml_conv_prepack_bytes",
+                            "b200ml_gemm_prepack_bytes"):
                 fn.restype = ctypes.c_int
         if path is None:
             _lib = lib

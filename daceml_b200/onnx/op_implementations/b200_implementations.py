@@ -68,8 +68,23 @@ def _b_is_constant(node, state, sdfg, conn="B"):
     return False
 
 
+def _prepacked_gemm_operand(node, state, sdfg, plan, b_layout, a_layout=0):
+    """A constant fp32 B is split into its TF32 parts once, here (``b200ml_gemm_prepack``); None when there is nothing to
+    prepare (no device, another type, B arrives at run time, or the product takes B as it is)."""
+    if not torch.cuda.is_available() or plan["batch"] != 1 or not _b_is_constant(node, state, sdfg):
+        return None
+    for e in state.in_edges_by_connector(node, "B"):
+        t = sdfg.constants[e.data.data]
+        if t.dtype != torch.float32:
+            return None
+        if not t.is_cuda:
+            t = t.to(torch.device("cuda", torch.cuda.current_device()))
+        return K.gemm_prepack(t.contiguous(), n=plan["n"], k=plan["k"], m=plan["m"], b_layout=b_layout, a_layout=a_layout)
+    return None
+
+
 def _launch_gemm(a, b, out, plan, *, b_layout=0, a_layout=0, alpha=1.0, bias=None, bias_scale=1.0, residual=None,
-                 residual_scale=1.0, act=0, ln=None, b_constant=False):
+                 residual_scale=1.0, act=0, ln=None, b_constant=False, packed=None):
     ctx = L.get_context(a.device)
     p = L.GemmParams()
     p.dtype = L.dtype_code(a.dtype)
@@ -95,7 +110,9 @@ def _launch_gemm(a, b, out, plan, *, b_layout=0, a_layout=0, alpha=1.0, bias=Non
         p.ln_gamma = ln[0].data_ptr() if ln[0] is not None else None
         p.ln_beta = ln[1].data_ptr() if ln[1] is not None else None
         p.ln_eps = ln[2]
-    K.gemm_raw(ctx, p, L.current_stream(a.device))
+    if packed is not None and packed.device != a.device:
+        packed = None
+    K.gemm_raw(ctx, p, L.current_stream(a.device), packed)
 
 
 @op_implementation(op="MatMul", name="b200")
@@ -112,9 +129,10 @@ class B200MatMul(ONNXForward):
         a, b = in_desc_with_name(node, state, sdfg, "A"), in_desc_with_name(node, state, sdfg, "B")
         plan = _matmul_plan(a.shape, b.shape)
         bc = _b_is_constant(node, state, sdfg)
+        packed = _prepacked_gemm_operand(node, state, sdfg, plan, 0)
 
         def run(ins, outs):
-            _launch_gemm(ins["A"], ins["B"], outs["Y"], plan, b_constant=bc)
+            _launch_gemm(ins["A"], ins["B"], outs["Y"], plan, b_constant=bc, packed=packed)
 
         return KernelTasklet(node.label, run, kernels=("gemm",))
 
@@ -149,10 +167,11 @@ class B200Gemm(ONNXForward):
         mode = B200Gemm._c_mode(node, state, sdfg)
         alpha, beta = float(node.alpha), float(node.beta)
         bc = _b_is_constant(node, state, sdfg)
+        packed = _prepacked_gemm_operand(node, state, sdfg, plan, tb, ta)
 
         def run(ins, outs):
             c = ins.get("C") if mode != "none" else None
-            _launch_gemm(ins["A"], ins["B"], outs["Y"], plan, a_layout=ta, b_layout=tb, alpha=alpha, b_constant=bc,
+            _launch_gemm(ins["A"], ins["B"], outs["Y"], plan, a_layout=ta, b_layout=tb, alpha=alpha, b_constant=bc, packed=packed,
                          bias=c if mode == "bias" else None, bias_scale=beta,
                          residual=c if mode == "full" else None, residual_scale=beta)
 
@@ -739,11 +758,12 @@ class B200FusedMatMul(ONNXForward):
         plan = dict(batch=1, m=prod(a.shape[:-1]), k=k, n=n, a_batched=False, b_batched=False)
         act, alpha = _ACT[node.activation], float(node.alpha)
         bc = _b_is_constant(node, state, sdfg)
+        packed = _prepacked_gemm_operand(node, state, sdfg, plan, tb)
         if node.ln_epsilon is None:
 
             def run(ins, outs):
                 _launch_gemm(ins["A"], ins["B"], outs["Y"], plan, b_layout=tb, alpha=alpha, bias=ins.get("Bias"),
-                             residual=ins.get("Residual"), act=act, b_constant=bc)
+                             residual=ins.get("Residual"), act=act, b_constant=bc, packed=packed)
 
             return KernelTasklet(node.label, run, kernels=("gemm",))
 
@@ -765,7 +785,7 @@ class B200FusedMatMul(ONNXForward):
         def run_split(ins, outs):
             y, tmp = outs["Y"], outs[pre]
             _launch_gemm(ins["A"], ins["B"], tmp, plan, b_layout=tb, alpha=alpha, bias=ins.get("Bias"),
-                         residual=ins.get("Residual"), act=act, b_constant=bc)
+                         residual=ins.get("Residual"), act=act, b_constant=bc, packed=packed)
             K.layernorm(tmp, y, gamma=ins.get("LnScale"), beta=ins.get("LnBias"), eps=eps)
 
         return KernelTasklet(node.label, run_split, kernels=("gemm", "layernorm"))

@@ -16,7 +16,7 @@ from . import lib as L
 # entry points in the order of the PlanOp enumeration; 'i' integer, 'f' float, 'p' address, 's' structure by
 # reference, 'a' array of numbers, 'q' array of addresses (the arguments between the context and the stream)
 _CALLS = [
-    ("b200ml_gemm", "s"), ("b200ml_softmax", "ipppiiifi"), ("b200ml_layernorm", "ippppppiif"), ("b200ml_reduce", "iippiii"),
+    ("b200ml_gemm_packed", "sp"), ("b200ml_softmax", "ipppiiifi"), ("b200ml_layernorm", "ippppppiif"), ("b200ml_reduce", "iippiii"),
     ("b200ml_unary", "iippiff"), ("b200ml_binary", "iipppiaaa"), ("b200ml_bias_act", "ippppiii"), ("b200ml_transpose", "ippiaa"),
     ("b200ml_cast", "iippi"), ("b200ml_conv2d", "s"), ("b200ml_se_gate", "ippppppiii"), ("b200ml_attention_f16", "s"),
     ("b200ml_strided_copy", "ippiaaa"), ("b200ml_strided_copy_parts", "iiqqiaaa"), ("b200ml_gather", "ipppiiii"),

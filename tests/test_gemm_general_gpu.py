@@ -1,0 +1,92 @@
+"""The fp32 tensor-core GEMM that splits its operands itself, and the kernel for a few rows: every operand layout, unaligned
+and ragged sizes, tiles of each width, K split over clusters (also with shares that are empty), batches, a packed B."""
+import ctypes
+
+import pytest
+import torch
+
+from daceml_b200 import kernels as K
+from daceml_b200 import lib as L
+
+pytestmark = pytest.mark.gpu
+
+# (m, n, k): one row to more than one tile; widths of the 32-, 64- and 128-column tiles; k of less than a k-block, of shares
+# that do not fill eight CTAs, of many blocks
+SIZES = [(1, 1, 1), (1, 120, 784), (3, 10, 33), (8, 17, 576), (9, 33, 100), (32, 64, 257), (33, 5, 31), (64, 100, 345), (127, 65, 129),
+         (129, 129, 97), (200, 32, 1000), (256, 300, 2052), (1000, 42, 826), (513, 10, 32)]
+
+
+def _turned(t):
+    return torch.empty(t.shape[1], t.shape[0], dtype=t.dtype, device=t.device).copy_(t.t())
+
+
+def _check(y, a, b, bias, dtype):
+    ref = a.double() @ b.double()
+    scale = a.double().abs() @ b.double().abs() + bias.double().abs()
+    ref = torch.relu(ref + bias.double())
+    # 22 bits of each operand, fp32 sums: the bound the split tensor-core products are held to; a half result adds its rounding
+    bound = 2e-6 * scale + (2.0**-10 * ref.abs() + 1e-7 if dtype == torch.float16 else 0.0)
+    err = (y.double() - ref).abs()
+    assert bool((err <= bound).all()), "worst error / bound %.3g" % float((err / bound).max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("a_layout, b_layout", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_general_gemm(dtype, a_layout, b_layout):
+    gen = torch.Generator("cuda").manual_seed(7)
+    for m, n, k in SIZES:
+        a = torch.randn(m, k, device="cuda", generator=gen).to(dtype)
+        b = (torch.randn(k, n, device="cuda", generator=gen) * 0.1).to(dtype)
+        bias = torch.randn(n, device="cuda", generator=gen).to(dtype)
+        guard = torch.full((m + 3, n), 7.0, dtype=dtype, device="cuda")
+        K.gemm(_turned(a) if a_layout else a, _turned(b) if b_layout else b, guard[:m], a_layout=a_layout, b_layout=b_layout,
+               bias=bias, act=L.EPI_RELU)
+        _check(guard[:m], a, b, bias, dtype)
+        assert bool((guard[m:] == 7.0).all()), "rows past M were written (%d x %d x %d)" % (m, n, k)
+    assert L.get_context(0).device_status() == 0
+
+
+@pytest.mark.parametrize("b_layout", [0, 1])
+def test_packed_operand_gives_the_same_product(b_layout):
+    gen = torch.Generator("cuda").manual_seed(8)
+    for m, n, k in [(40, 10, 32), (33, 120, 785), (130, 33, 64), (300, 257, 100), (4096, 32, 120)]:
+        a, b = torch.randn(m, k, device="cuda", generator=gen), torch.randn(k, n, device="cuda", generator=gen) * 0.1
+        bias = torch.randn(n, device="cuda", generator=gen)
+        bl = _turned(b) if b_layout else b
+        packed = K.gemm_prepack(bl, n=n, k=k, m=m, b_layout=b_layout)
+        assert packed is not None
+        y = torch.empty(m, n, device="cuda")
+        p = L.GemmParams()
+        p.dtype, p.b_layout, p.epilogue, p.alpha, p.bias_scale = L.F32, b_layout, L.EPI_BIAS | L.EPI_RELU, 1.0, 1.0
+        p.m, p.n, p.k, p.batch_outer, p.batch_inner, p.lda, p.ldb, p.ldc = m, n, k, 1, 1, k, k if b_layout else n, n
+        p.a, p.b, p.c, p.bias, p.flags = a.data_ptr(), bl.data_ptr(), y.data_ptr(), bias.data_ptr(), L.GEMM_B_CONSTANT
+        ctx = L.get_context(0)
+        L.check(ctx.lib.b200ml_gemm_packed(ctx.handle, ctypes.byref(p), L.ptr(packed), L.current_stream()))
+        _check(y, a, b, bias, torch.float32)
+    assert L.get_context(0).device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_batched_general_gemm(dtype):
+    gen = torch.Generator("cuda").manual_seed(9)
+    for m, n, k, b_layout in [(5, 37, 64, 1), (77, 77, 64, 1), (130, 64, 77, 0), (40, 9, 33, 1)]:
+        a = torch.randn(2, 3, m, k, device="cuda", generator=gen).to(dtype)
+        b = torch.randn(2, 3, k, n, device="cuda", generator=gen).to(dtype)
+        y = torch.empty(2, 3, m, n, dtype=dtype, device="cuda")
+        K.gemm_batched(a, b.transpose(2, 3).contiguous() if b_layout else b, y, b_layout=b_layout, act=L.EPI_RELU)
+        for i in range(6):
+            _check(y.view(6, m, n)[i], a.view(6, m, k)[i], b.view(6, k, n)[i], torch.zeros(n, device="cuda"), dtype)
+    assert L.get_context(0).device_status() == 0
+
+
+@pytest.mark.parametrize("m, n, k, a_layout", [(4749, 513, 100, 0), (4096, 640, 36, 1), (20000, 400, 1100, 0)])
+def test_products_of_many_tiles_pack_both_operands(m, n, k, a_layout):
+    """Ragged sizes with more tiles than SMs; the last one takes its rows in pieces (its packed form exceeds the workspace)."""
+    gen = torch.Generator("cuda").manual_seed(10)
+    a, b = torch.randn(m, k, device="cuda", generator=gen), torch.randn(k, n, device="cuda", generator=gen) * 0.1
+    bias = torch.randn(n, device="cuda", generator=gen)
+    y = torch.full((m + 3, n), 7.0, device="cuda")
+    K.gemm(_turned(a) if a_layout else a, b, y[:m], a_layout=a_layout, bias=bias, act=L.EPI_RELU)
+    _check(y[:m], a, b, bias, torch.float32)
+    assert bool((y[m:] == 7.0).all())
+    assert L.get_context(0).device_status() == 0
