@@ -57,6 +57,7 @@ int transpose(const b200ml_ctx* ctx, int elem_bytes, const void* x, void* y, int
 int cast(const b200ml_ctx* ctx, int src, int dst, const void* x, void* y, int64_t n, cudaStream_t s);
 int cast_any(const b200ml_ctx* ctx, int src, int dst, const void* x, void* y, int64_t n, cudaStream_t s);
 int conv2d(const b200ml_ctx* ctx, const b200ml_conv_params* p, cudaStream_t s);
+int32_t conv_channels_last(const b200ml_ctx* ctx, const b200ml_conv_params* p);
 int64_t conv_prepack_bytes(const b200ml_ctx* ctx, const b200ml_conv_params* p);
 int conv_prepack(const b200ml_ctx* ctx, const b200ml_conv_params* p, void* packed, cudaStream_t s);
 int se_gate(const b200ml_ctx* ctx, int dtype, const void* pooled, const void* w1, const void* b1, const void* w2,
@@ -97,12 +98,15 @@ thread_local int64_t t_tmap_hits = 0, t_tmap_misses = 0;
 
 CUresult encode_tiled_cached(const b200ml_ctx* ctx, CUtensorMap* out, CUtensorMapDataType dtype, const void* base,
                              const cuuint64_t dims[4], const cuuint64_t strides[3], const cuuint32_t box[4],
-                             CUtensorMapSwizzle swizzle) {
+                             CUtensorMapSwizzle swizzle, const cuuint32_t* element_strides) {
     EncodeTiledFn fn = reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled);
     if (!fn) return CUDA_ERROR_NOT_SUPPORTED;
     TmapKey key;
     key.w[0] = reinterpret_cast<uint64_t>(base);
-    key.w[1] = static_cast<uint64_t>(dtype) | (static_cast<uint64_t>(swizzle) << 16) | (static_cast<uint64_t>(ctx->device) << 32);
+    key.w[1] = static_cast<uint64_t>(dtype) | (static_cast<uint64_t>(swizzle) << 8) | (static_cast<uint64_t>(ctx->device) << 32);
+    const cuuint32_t unit[4] = {1, 1, 1, 1};
+    const cuuint32_t* estr = element_strides ? element_strides : unit;
+    for (int i = 0; i < 4; ++i) key.w[1] |= static_cast<uint64_t>(estr[i] & 15u) << (16 + 4 * i);
     for (int i = 0; i < 4; ++i) key.w[2 + i] = dims[i];
     for (int i = 0; i < 3; ++i) key.w[6 + i] = strides[i];
     for (int i = 0; i < 4; ++i) key.w[9 + i] = box[i];
@@ -116,7 +120,6 @@ CUresult encode_tiled_cached(const b200ml_ctx* ctx, CUtensorMap* out, CUtensorMa
         return CUDA_SUCCESS;
     }
     ++t_tmap_misses;
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = fn(out, dtype, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r == CUDA_SUCCESS && e) {
@@ -365,8 +368,13 @@ int b200ml_cast(b200ml_ctx* ctx, int32_t src_dtype, int32_t dst_dtype, const voi
 }
 
 int64_t b200ml_conv_prepack_bytes(b200ml_ctx* ctx, const b200ml_conv_params* p) {
-    if (ctx == nullptr || p == nullptr || p->dtype != B200ML_F32) return 0;
+    if (ctx == nullptr || p == nullptr || !dtype_ok(p->dtype)) return 0;
     return conv_prepack_bytes(ctx, p);
+}
+
+int32_t b200ml_conv_channels_last(b200ml_ctx* ctx, const b200ml_conv_params* p) {
+    if (ctx == nullptr || p == nullptr || !dtype_ok(p->dtype)) return 0;
+    return conv_channels_last(ctx, p);
 }
 
 int b200ml_conv_prepack(b200ml_ctx* ctx, const b200ml_conv_params* p, void* packed, b200ml_stream stream) {

@@ -96,7 +96,6 @@ attention_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     uint64_t* o_final = p_full + NC;            // [NC] every product of the chain has finished
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_final + NC);
 
-    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int qblk = blockIdx.x % args.q_blocks;
@@ -132,6 +131,7 @@ attention_f16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     }
     ptx::tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();  // after the allocation: an early CTA of the next kernel cannot take this CTA's tensor memory
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();  // everything above overlaps the previous kernel's tail

@@ -13,6 +13,10 @@ namespace b200ml {
 
 int reduce(const b200ml_ctx* ctx, int dtype, int op, const void* x, void* y, int64_t outer, int64_t red, int64_t inner,
            cudaStream_t s);
+bool conv_f16_applies(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow);
+int64_t conv_f16_pack_bytes(const b200ml_conv_params* p);
+int conv_f16_pack(const b200ml_ctx* ctx, const b200ml_conv_params* p, void* packed, cudaStream_t s);
+int conv_f16(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow, cudaStream_t s);
 bool conv1x1_tensor_core_applies(const b200ml_ctx* ctx, const b200ml_conv_params* p);
 int conv1x1_tensor_core(const b200ml_ctx* ctx, const b200ml_conv_params* p, cudaStream_t stream);
 bool conv_igemm_applies(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow);
@@ -26,6 +30,26 @@ namespace {
 
 __device__ __forceinline__ float ldv(const float* p) { return __ldg(p); }
 __device__ __forceinline__ float ldv(const __half* p) { return __half2float(__ldg(p)); }
+// Four adjacent values of either type at once.
+template <typename T>
+struct Vec4;
+template <>
+struct Vec4<float> { using type = float4; };
+template <>
+struct Vec4<__half> { using type = uint2; };
+__device__ __forceinline__ float4 ldv4(const float4* p) { return __ldg(p); }
+__device__ __forceinline__ float4 ldv4(const uint2* p) {
+    const uint2 q = __ldg(p);
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&q.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void stv4(float4* p, const float4& v) { *p = v; }
+__device__ __forceinline__ void stv4(uint2* p, const float4& v) {
+    uint2 q;
+    *reinterpret_cast<__half2*>(&q.x) = __floats2half2_rn(v.x, v.y);
+    *reinterpret_cast<__half2*>(&q.y) = __floats2half2_rn(v.z, v.w);
+    *p = q;
+}
 __device__ __forceinline__ void stv(float* p, float v) { *p = v; }
 __device__ __forceinline__ void stv(__half* p, float v) { *p = __float2half_rn(v); }
 
@@ -293,35 +317,36 @@ __global__ void __launch_bounds__(128) pointwise_acc_kernel(const float* __restr
 // ---------------------------------------------------------------------------------------------
 // depthwise convolution, stride 1: one (image, channel) plane per block
 // ---------------------------------------------------------------------------------------------
-// 3x3, unit stride and dilation, planes up to 64 pixels wide: no shared memory.  A lane owns one output column of a
+// 3x3, unit stride and dilation: no shared memory.  A lane owns one output column of a
 // strip of rows and slides a 3x3 window down it - three (L1-served) loads, nine multiply-adds, one store per output,
 // against the 130 instructions per output of the staged kernel below (index arithmetic and shared-memory traffic).
-__global__ void __launch_bounds__(256) depthwise3x3_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                           const float* __restrict__ bias, float* __restrict__ y,
-                                                           float* __restrict__ pool_mean, const ConvGeom g) {
+template <typename T>
+__global__ void __launch_bounds__(256) depthwise3x3_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias,
+                                                           T* __restrict__ y, T* __restrict__ pool_mean, const ConvGeom g) {
     __shared__ float red[8];
     const int ch = blockIdx.x % g.c;
     const int64_t img = blockIdx.x / g.c;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float* xp = x + (img * g.c + ch) * static_cast<int64_t>(g.h) * g.w;
-    float* yp = y + (img * g.m + ch) * static_cast<int64_t>(g.oh) * g.ow;
+    const T* xp = x + (img * g.c + ch) * static_cast<int64_t>(g.h) * g.w;
+    T* yp = y + (img * g.m + ch) * static_cast<int64_t>(g.oh) * g.ow;
     float t[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) t[i] = __ldg(w + ch * 9 + i);
-    const float b = bias ? __ldg(bias + ch) : 0.0f;
-    const int ox = lane + 32 * (warp & 1);
-    const bool col_ok = ox < g.ow;
+    for (int i = 0; i < 9; ++i) t[i] = ldv(w + ch * 9 + i);
+    const float b = bias ? ldv(bias + ch) : 0.0f;
     const int rows_per = (g.oh + 3) >> 2;  // four strips of rows
     const int oy0 = (warp >> 1) * rows_per;
     const int oy1 = oy0 + rows_per < g.oh ? oy0 + rows_per : g.oh;
+    float local = 0.0f;
+    for (int ox = lane + 32 * (warp & 1); ox < ((g.ow + 63) & ~63); ox += 64) {  // 64 columns at a time
+    const bool col_ok = ox < g.ow;
     const int ix0 = ox - g.pl;
     auto load_row = [&](int iy, float (&v)[3]) {
         const bool row_in = col_ok && iy >= 0 && iy < g.h;
-        const float* rp = xp + static_cast<int64_t>(iy) * g.w;
+        const T* rp = xp + static_cast<int64_t>(iy) * g.w;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             const int ix = ix0 + j;
-            v[j] = (row_in && ix >= 0 && ix < g.w) ? __ldg(rp + ix) : 0.0f;
+            v[j] = (row_in && ix >= 0 && ix < g.w) ? ldv(rp + ix) : 0.0f;
         }
     };
     // four output rows per step: the twelve loads of the next four input rows are issued before the first
@@ -329,7 +354,6 @@ __global__ void __launch_bounds__(256) depthwise3x3_kernel(const float* __restri
     float r[6][3];
     load_row(oy0 - g.pt, r[0]);
     load_row(oy0 - g.pt + 1, r[1]);
-    float local = 0.0f;
     for (int oy = oy0; oy < oy1; oy += 4) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) load_row(oy + k - g.pt + 2, r[2 + k]);
@@ -342,12 +366,13 @@ __global__ void __launch_bounds__(256) depthwise3x3_kernel(const float* __restri
                 for (int j = 0; j < 3; ++j) acc = fmaf(t[i * 3 + j], r[k + i][j], acc);
             acc = conv_act(acc, g.act);
             if (col_ok && oy + k < oy1) {
-                yp[(oy + k) * g.ow + ox] = acc;
+                stv(yp + (oy + k) * g.ow + ox, acc);
                 local += acc;
             }
         }
 #pragma unroll
         for (int j = 0; j < 3; ++j) r[0][j] = r[4][j], r[1][j] = r[5][j];
+    }
     }
     if (pool_mean) {
 #pragma unroll
@@ -357,20 +382,19 @@ __global__ void __launch_bounds__(256) depthwise3x3_kernel(const float* __restri
         if (threadIdx.x == 0) {
             float tot = 0.0f;
             for (int i = 0; i < 8; ++i) tot += red[i];
-            pool_mean[img * g.m + ch] = tot / (g.oh * g.ow);
+            stv(pool_mean + img * g.m + ch, tot / (g.oh * g.ow));
         }
     }
 }
 
-// 3x3, unit stride, pad 1 on every side, width a multiple of 4 up to 64: a lane owns FOUR adjacent output columns of a
+// 3x3, unit stride, pad 1 on every side, width a multiple of 4 up to 128: a lane owns FOUR adjacent output columns of a
 // strip of rows.  Per input row it issues one 16-byte load; the two halo columns come from the neighbouring lanes by
 // shuffle (zero at the plane's edges), so four outputs cost one load, two shuffles, 36 multiply-adds and one 16-byte
 // store - a quarter of the instructions of the column-per-lane kernel above, which is bound by instruction issue.
 // One warp per plane: LPR = w / 4 lanes cover a row, 32 / LPR strips of rows share the warp.
-__global__ void __launch_bounds__(128) depthwise3x3_quad_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                                const float* __restrict__ bias, float* __restrict__ y,
-                                                                float* __restrict__ pool_mean, const ConvGeom g,
-                                                                int64_t planes) {
+template <typename T>
+__global__ void __launch_bounds__(128) depthwise3x3_quad_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias,
+                                                                T* __restrict__ y, T* __restrict__ pool_mean, const ConvGeom g, int64_t planes) {
     const int lane = threadIdx.x & 31;
     const int64_t plane = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (plane >= planes) return;  // whole warps leave; no block-wide barrier below
@@ -383,17 +407,18 @@ __global__ void __launch_bounds__(128) depthwise3x3_quad_kernel(const float* __r
     const int rows_per = (g.h + strips - 1) / strips;
     const int oy0 = strip * rows_per;
     const int oy1 = active ? (oy0 + rows_per < g.h ? oy0 + rows_per : g.h) : oy0;
-    const float4* xp = reinterpret_cast<const float4*>(x + (img * g.c + ch) * static_cast<int64_t>(g.h) * g.w) + q;
-    float4* yp = reinterpret_cast<float4*>(y + (img * g.m + ch) * static_cast<int64_t>(g.h) * g.w) + q;
+    using V = typename Vec4<T>::type;
+    const V* xp = reinterpret_cast<const V*>(x + (img * g.c + ch) * static_cast<int64_t>(g.h) * g.w) + q;
+    V* yp = reinterpret_cast<V*>(y + (img * g.m + ch) * static_cast<int64_t>(g.h) * g.w) + q;
     float t[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) t[i] = __ldg(w + ch * 9 + i);
-    const float b = bias ? __ldg(bias + ch) : 0.0f;
+    for (int i = 0; i < 9; ++i) t[i] = ldv(w + ch * 9 + i);
+    const float b = bias ? ldv(bias + ch) : 0.0f;
 
     // a row as this lane sees it: left halo, four own columns, right halo
     struct Row { float v[6]; };
     auto fetch = [&](int iy) -> float4 {
-        return (active && iy >= 0 && iy < g.h) ? __ldg(xp + static_cast<int64_t>(iy) * lpr) : make_float4(0.f, 0.f, 0.f, 0.f);
+        return (active && iy >= 0 && iy < g.h) ? ldv4(xp + static_cast<int64_t>(iy) * lpr) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     auto finish = [&](const float4& c) -> Row {
         Row r;
@@ -430,12 +455,12 @@ __global__ void __launch_bounds__(128) depthwise3x3_quad_kernel(const float* __r
         const Row rc = finish(c0), rd = finish(c1);
         if (oy < oy1) {
             const float4 o = output(ra, rb, rc);
-            yp[static_cast<int64_t>(oy) * lpr] = o;
+            stv4(yp + static_cast<int64_t>(oy) * lpr, o);
             local += (o.x + o.y) + (o.z + o.w);
         }
         if (oy + 1 < oy1) {
             const float4 o = output(rb, rc, rd);
-            yp[static_cast<int64_t>(oy + 1) * lpr] = o;
+            stv4(yp + static_cast<int64_t>(oy + 1) * lpr, o);
             local += (o.x + o.y) + (o.z + o.w);
         }
         ra = rc, rb = rd;
@@ -443,15 +468,15 @@ __global__ void __launch_bounds__(128) depthwise3x3_quad_kernel(const float* __r
     if (pool_mean) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-        if (lane == 0) pool_mean[img * g.m + ch] = local / (g.h * g.w);
+        if (lane == 0) stv(pool_mean + img * g.m + ch, local / (g.h * g.w));
     }
 }
 
 // Any kernel size up to 64 taps: the plane and its halo staged in shared memory.  Warps walk rows and lanes walk
 // columns, so no index needs a division.
-__global__ void __launch_bounds__(256) depthwise_plane_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                              const float* __restrict__ bias, float* __restrict__ y,
-                                                              float* __restrict__ pool_mean, const ConvGeom g) {
+template <typename T>
+__global__ void __launch_bounds__(256) depthwise_plane_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias,
+                                                              T* __restrict__ y, T* __restrict__ pool_mean, const ConvGeom g) {
     extern __shared__ float plane[];  // (h + kh - 1 ... ) padded input plane
     __shared__ float red[8];
     __shared__ float wk[64];
@@ -460,19 +485,19 @@ __global__ void __launch_bounds__(256) depthwise_plane_kernel(const float* __res
     const int kh = g.kh, kw = g.kw;
     const int ph = g.oh + kh - 1, pw = g.ow + kw - 1;  // padded plane extents actually read
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float* xp = x + (img * g.c + ch) * static_cast<int64_t>(g.h) * g.w;
+    const T* xp = x + (img * g.c + ch) * static_cast<int64_t>(g.h) * g.w;
     for (int py = warp; py < ph; py += 8) {
         const int iy = py - g.pt;
         const bool row_in = iy >= 0 && iy < g.h;
         for (int px = lane; px < pw; px += 32) {
             const int ix = px - g.pl;
-            plane[py * pw + px] = (row_in && ix >= 0 && ix < g.w) ? __ldg(xp + iy * g.w + ix) : 0.0f;
+            plane[py * pw + px] = (row_in && ix >= 0 && ix < g.w) ? ldv(xp + iy * g.w + ix) : 0.0f;
         }
     }
-    if (threadIdx.x < kh * kw) wk[threadIdx.x] = __ldg(w + ch * kh * kw + threadIdx.x);
+    if (threadIdx.x < kh * kw) wk[threadIdx.x] = ldv(w + ch * kh * kw + threadIdx.x);
     __syncthreads();
-    const float b = bias ? __ldg(bias + ch) : 0.0f;
-    float* yp = y + (img * g.m + ch) * static_cast<int64_t>(g.oh) * g.ow;
+    const float b = bias ? ldv(bias + ch) : 0.0f;
+    T* yp = y + (img * g.m + ch) * static_cast<int64_t>(g.oh) * g.ow;
     float local = 0.0f;
     for (int oy = warp; oy < g.oh; oy += 8) {
         for (int ox = lane; ox < g.ow; ox += 32) {
@@ -480,7 +505,7 @@ __global__ void __launch_bounds__(256) depthwise_plane_kernel(const float* __res
             for (int i = 0; i < kh; ++i)
                 for (int j = 0; j < kw; ++j) acc = fmaf(wk[i * kw + j], plane[(oy + i) * pw + ox + j], acc);
             acc = conv_act(acc, g.act);
-            yp[oy * g.ow + ox] = acc;
+            stv(yp + oy * g.ow + ox, acc);
             local += acc;
         }
     }
@@ -492,7 +517,7 @@ __global__ void __launch_bounds__(256) depthwise_plane_kernel(const float* __res
         if (threadIdx.x == 0) {
             float tot = 0.0f;
             for (int i = 0; i < 8; ++i) tot += red[i];
-            pool_mean[img * g.m + ch] = tot / (g.oh * g.ow);
+            stv(pool_mean + img * g.m + ch, tot / (g.oh * g.ow));
         }
     }
 }
@@ -547,12 +572,40 @@ int launch_direct(const b200ml_conv_params* p, const ConvGeom& g, cudaStream_t s
 
 }  // namespace
 
+// Depthwise, stride 1 (either type): what the shape allows of the three kernels above.
+template <typename T>
+static int depthwise_fast(const b200ml_conv_params* p, const ConvGeom& g, cudaStream_t s, bool* launched, bool* pooled) {
+    const bool unit = p->stride_h == 1 && p->stride_w == 1 && p->dil_h == 1 && p->dil_w == 1;
+    const int64_t planes = p->n * p->c;
+    if (!unit || p->group != p->c || p->m != p->c || p->gate || p->residual || p->kh * p->kw > 64 || planes >= (1ll << 31)) return B200ML_OK;
+    const T *x = (const T*)p->x, *w = (const T*)p->weight, *b = (const T*)p->bias;
+    T *y = (T*)p->y, *pool = reinterpret_cast<T*>(p->pool_sum);
+    const bool pad1 = p->pad_top == 1 && p->pad_left == 1 && p->pad_bottom == 1 && p->pad_right == 1;
+    const size_t sm = (size_t)(g.oh + p->kh - 1) * (g.ow + p->kw - 1) * sizeof(float);
+    const bool three = p->kh == 3 && p->kw == 3;
+    if (three && pad1 && p->w % 4 == 0 && p->w >= 8 && p->w <= 128 && aligned16(x) && aligned16(y))
+        depthwise3x3_quad_kernel<T><<<(unsigned)ceil_div(planes, 4), 128, 0, s>>>(x, w, b, y, pool, g, planes);
+    else if (three) depthwise3x3_kernel<T><<<(unsigned)planes, 256, 0, s>>>(x, w, b, y, pool, g);
+    else if (sm <= 40 * 1024) depthwise_plane_kernel<T><<<(unsigned)planes, 256, sm, s>>>(x, w, b, y, pool, g);
+    else return B200ML_OK;
+    *launched = true;
+    *pooled = true;
+    return check_launch("depthwise");
+}
+
 // Tries the specialised kernels; *launched says whether one ran, *pooled whether it also wrote the pool.
 static int conv2d_fast(const b200ml_ctx* ctx, const b200ml_conv_params* p, const ConvGeom& g, cudaStream_t s, bool* launched,
                        bool* pooled) {
     *launched = false;
     *pooled = false;
-    if (p->dtype != B200ML_F32) return B200ML_OK;
+    if (conv_f16_applies(ctx, p, g.oh, g.ow)) {  // fp16, group 1: implicit GEMM on the tensor core over channels-last operands
+        *launched = true;
+        return conv_f16(ctx, p, g.oh, g.ow, s);
+    }
+    if (p->act & (B200ML_CONV_X_NHWC | B200ML_CONV_Y_NHWC))
+        return fail(B200ML_ERR_UNSUPPORTED, "conv: channels-last tensors need a convolution the fp16 tensor-core kernel takes");
+    int rc = p->dtype == B200ML_F32 ? depthwise_fast<float>(p, g, s, launched, pooled) : depthwise_fast<__half>(p, g, s, launched, pooled);
+    if (rc || *launched || p->dtype != B200ML_F32) return rc;
     if (conv1x1_tensor_core_applies(ctx, p)) {  // 1x1, stride 1: the tensor-core kernel (3 x TF32), HBM-bound
         *launched = true;
         return conv1x1_tensor_core(ctx, p, s);
@@ -617,20 +670,6 @@ static int conv2d_fast(const b200ml_ctx* ctx, const b200ml_conv_params* p, const
             }
         }
     }
-    if (unit && p->group == p->c && p->m == p->c && !gt && !r && p->kh * p->kw <= 64) {
-        const size_t sm = (size_t)(g.oh + p->kh - 1) * (g.ow + p->kw - 1) * sizeof(float);
-        if (sm <= 40 * 1024 && p->n * p->c < (1ll << 31)) {
-            const bool pad1 = p->pad_top == 1 && p->pad_left == 1 && p->pad_bottom == 1 && p->pad_right == 1;
-            if (p->kh == 3 && p->kw == 3 && pad1 && p->w % 4 == 0 && p->w >= 8 && p->w <= 64 && aligned16(x) && aligned16(y)) {
-                const int64_t planes = p->n * p->c;
-                depthwise3x3_quad_kernel<<<(unsigned)ceil_div(planes, 4), 128, 0, s>>>(x, w, b, y, p->pool_sum, g, planes);
-            } else if (p->kh == 3 && p->kw == 3 && g.ow <= 64) depthwise3x3_kernel<<<(unsigned)(p->n * p->c), 256, 0, s>>>(x, w, b, y, p->pool_sum, g);
-            else depthwise_plane_kernel<<<(unsigned)(p->n * p->c), 256, sm, s>>>(x, w, b, y, p->pool_sum, g);
-            *launched = true;
-            *pooled = true;
-            return check_launch("depthwise_plane");
-        }
-    }
     return B200ML_OK;
 }
 
@@ -660,7 +699,8 @@ int conv2d(const b200ml_ctx* ctx, const b200ml_conv_params* p, cudaStream_t s) {
     return B200ML_OK;
 }
 
-// Which tensor-core kernel (if any) takes this convolution: 1 = the 1x1 kernel, 2 = the implicit GEMM, 0 = neither.
+// Which tensor-core kernel (if any) takes this convolution: 1 = the 1x1 kernel, 2 = the fp32 implicit GEMM, 3 = the fp16 one,
+// 0 = none.
 static int conv_tensor_core_kind(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t* ow_out) {
     if (p->group < 1 || p->stride_h < 1 || p->stride_w < 1 || p->dil_h < 1 || p->dil_w < 1 || p->kh < 1 || p->kw < 1) return 0;
     const int64_t eh = p->h + p->pad_top + p->pad_bottom - p->dil_h * (p->kh - 1) - 1;
@@ -672,15 +712,22 @@ static int conv_tensor_core_kind(const b200ml_ctx* ctx, const b200ml_conv_params
     b200ml_conv_params q = *p;
     if (!q.x) q.x = reinterpret_cast<const void*>(uintptr_t(256));
     if (!q.y) q.y = reinterpret_cast<void*>(uintptr_t(256));
+    if (conv_f16_applies(ctx, &q, oh, ow)) return 3;
     if (conv1x1_tensor_core_applies(ctx, &q)) return 1;
     if (conv_igemm_applies(ctx, &q, oh, ow)) return 2;
     return 0;
 }
 
+int32_t conv_channels_last(const b200ml_ctx* ctx, const b200ml_conv_params* p) {
+    int64_t ow = 0;
+    if (conv_tensor_core_kind(ctx, p, &ow) != 3 || p->pool_sum) return 0;
+    return (!(p->act & B200ML_CONV_X_NHWC) || (p->c % 8 == 0 && !p->gate)) && (!(p->act & B200ML_CONV_Y_NHWC) || p->m % 8 == 0) ? 1 : 0;
+}
+
 int64_t conv_prepack_bytes(const b200ml_ctx* ctx, const b200ml_conv_params* p) {
     int64_t ow = 0;
     const int kind = conv_tensor_core_kind(ctx, p, &ow);
-    return kind == 1 ? conv1x1_pack_bytes(p) : (kind == 2 ? conv_igemm_pack_bytes(p, ow) : 0);
+    return kind == 3 ? conv_f16_pack_bytes(p) : kind == 1 ? conv1x1_pack_bytes(p) : (kind == 2 ? conv_igemm_pack_bytes(p, ow) : 0);
 }
 
 int conv_prepack(const b200ml_ctx* ctx, const b200ml_conv_params* p, void* packed, cudaStream_t s) {
@@ -688,7 +735,7 @@ int conv_prepack(const b200ml_ctx* ctx, const b200ml_conv_params* p, void* packe
     const int kind = conv_tensor_core_kind(ctx, p, &ow);
     B200ML_REQUIRE(kind != 0, "conv_prepack: this convolution takes its weights as they are (b200ml_conv_prepack_bytes returns 0)");
     B200ML_REQUIRE(packed && aligned16(packed) && p->weight, "conv_prepack: the packed buffer must be 16-byte aligned device memory, the weights given");
-    return kind == 1 ? conv1x1_pack(ctx, p, packed, s) : conv_igemm_pack(ctx, p, ow, packed, s);
+    return kind == 3 ? conv_f16_pack(ctx, p, packed, s) : kind == 1 ? conv1x1_pack(ctx, p, packed, s) : conv_igemm_pack(ctx, p, ow, packed, s);
 }
 
 int se_gate(const b200ml_ctx*, int dtype, const void* pooled, const void* w1, const void* b1, const void* w2,

@@ -89,7 +89,6 @@ conv1x1_tf32x3_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     uint64_t* tmem_empty = tmem_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
-    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     uint32_t tmem_cols = 32;
@@ -122,6 +121,7 @@ conv1x1_tf32x3_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     }
     ptx::tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();  // after the allocation: an early CTA of the next kernel cannot take this CTA's tensor memory
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();  // the split weights (and possibly X, the gate, the residual) come from kernels before this one in the stream

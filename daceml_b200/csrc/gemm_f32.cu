@@ -41,7 +41,9 @@ struct F32Smem {
     static constexpr int PARTS = sizeof(T) == 4 ? 2 : 1;  // hi and lo; fp16 values have no lo part
     static constexpr int A_BYTES = FM * FK * 4, B_BYTES = BN * FK * 4;
     static constexpr int STAGE_BYTES = PARTS * (A_BYTES + B_BYTES);
-    static constexpr int STAGES = BN == 128 ? 3 : 4;
+    // As many as fit beside the barriers; more than half of an SM's shared memory in every case, so that no two CTAs - of one
+    // cluster, waiting for one another - can share an SM and wait for each other's tensor memory.
+    static constexpr int STAGES = BN == 128 ? 6 / PARTS : (PARTS == 1 ? 8 : 4);
     static constexpr int PART_LD = BN + 4;  // floats between rows of the parked tile: 16-byte rows, no bank conflicts
     static constexpr int TOTAL = STAGES * STAGE_BYTES + 256 + 1024;
     static_assert(FM * PART_LD * 4 <= STAGES * STAGE_BYTES, "the parked tile lies over the pipeline stages");
@@ -196,7 +198,6 @@ __global__ void __launch_bounds__(F_THREADS, 1) gemm_f32_kernel(const F32Args<T>
     uint64_t* acc_bar = empty_bar + STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
 
-    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = g.split > 1 ? static_cast<int>(ptx::cluster_ctarank()) : 0;
     const int tile = blockIdx.x / g.split;
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) gemm_f32_kernel(const F32Args<T>
     }
     ptx::tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();  // after the allocation: an early CTA of the next kernel cannot take this CTA's tensor memory
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 

@@ -46,7 +46,6 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     float* red = reinterpret_cast<float*>(smem + LN_STAGES * LN_STAGE_BYTES + 256);  // [4][128]: sum and sum of squares per column half
     float* stats = red + 4 * BM;                                                       // [2][128]: this CTA's row sum and sum of squares
 
-    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t rank = ptx::cluster_ctarank();
@@ -83,6 +82,7 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     }
     ptx::tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();  // after the allocation: an early CTA of the next kernel cannot take this CTA's tensor memory
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // A constant B (weights): its parts of the first stages are requested before the dependency wait (see gemm_tc.cu)

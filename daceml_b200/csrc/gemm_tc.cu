@@ -57,7 +57,6 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     uint64_t* tmem_empty_bar = tmem_full_bar + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
 
-    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int num_kb = (args.k + BK - 1) / BK;
@@ -85,6 +84,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     }
     ptx::tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();  // after the allocation: an early CTA of the next kernel cannot take this CTA's tensor memory
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // A constant B (weights) does not depend on the kernel in front of this one: the B parts of the first tile's first

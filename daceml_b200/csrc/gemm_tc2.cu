@@ -56,7 +56,6 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     uint64_t* tmem_empty_bar = tmem_full_bar + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
 
-    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t cta = ptx::cluster_ctarank();  // 0: leader (issues the MMAs), 1: peer
@@ -87,6 +86,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     }
     ptx::tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();  // after the allocation: an early CTA of the next kernel cannot take this CTA's tensor memory
     ptx::cluster_sync();  // both CTAs' barriers exist before any remote arrive or load completion
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;

@@ -340,7 +340,7 @@ def conv_prepack(x_shape, w, *, bias=None, strides=(1, 1), pads=(0, 0, 0, 0), di
     """Prepares constant convolution weights once (``b200ml_conv_prepack``): returns the packed tensor to pass to
     :func:`conv2d` as ``packed_weight``, or None when this convolution runs on a kernel that takes the weights as they
     are.  ``w`` and ``bias`` are device tensors; ``gate`` says whether the calls will carry a squeeze-excite gate."""
-    if not w.is_cuda or w.dtype != torch.float32:
+    if not w.is_cuda or w.dtype not in (torch.float32, torch.float16):
         return None
     ctx = _ctx(w)
     for t in (w, bias):
@@ -353,6 +353,24 @@ def conv_prepack(x_shape, w, *, bias=None, strides=(1, 1), pads=(0, 0, 0, 0), di
     packed = torch.empty(nbytes, dtype=torch.uint8, device=w.device)
     L.check(ctx.lib.b200ml_conv_prepack(ctx.handle, ctypes.byref(p), ctypes.c_void_p(packed.data_ptr()), _stream(w)))
     return packed
+
+
+def conv_channels_last(x_shape, dtype, w_shape, device, *, strides=(1, 1), pads=(0, 0, 0, 0), dilations=(1, 1), group=1, x_last=False,
+                       y_last=False):
+    """Whether this convolution can read X (``x_last``) and write Y (``y_last``) channels-last
+    (``b200ml_conv_channels_last``); the tensors keep their NCHW descriptors."""
+    if not torch.cuda.is_available() or dtype != torch.float16:
+        return False
+    ctx = L.get_context(device)
+    p = L.ConvParams()
+    p.dtype, p.act = L.F16, (L.CONV_X_NHWC if x_last else 0) | (L.CONV_Y_NHWC if y_last else 0)
+    p.n, p.c, p.h, p.w = x_shape
+    p.m, _, p.kh, p.kw = w_shape
+    p.stride_h, p.stride_w = strides
+    p.pad_top, p.pad_left, p.pad_bottom, p.pad_right = pads
+    p.dil_h, p.dil_w = dilations
+    p.group = group
+    return bool(ctx.lib.b200ml_conv_channels_last(ctx.handle, ctypes.byref(p)))
 
 
 def se_gate(pooled, w1, b1, w2, b2, out):

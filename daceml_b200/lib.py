@@ -20,6 +20,7 @@ OK, ERR_INVALID, ERR_UNSUPPORTED, ERR_CUDA, ERR_DEVICE, ERR_WORKSPACE = 0, -1, -
 F16, F32, I64, I32, F64, U8, BOOL = range(7)
 EPI_BIAS, EPI_RELU, EPI_GELU, EPI_RESIDUAL, EPI_SWISH, EPI_LAYERNORM = 1, 2, 4, 8, 16, 32
 GEMM_B_CONSTANT = 1
+CONV_X_NHWC, CONV_Y_NHWC = 256, 512
 RED_SUM, RED_MEAN, RED_MAX, RED_MIN = 0, 1, 2, 3
 (UN_COPY, UN_RELU, UN_SIGMOID, UN_ERF, UN_SQRT, UN_EXP, UN_LOG, UN_TANH, UN_SWISH, UN_GELU, UN_RECIPROCAL,
  UN_LEAKYRELU, UN_AFFINE, UN_POWS, UN_SOFTPLUS, UN_CLIP, UN_NEG, UN_ABS) = range(18)
@@ -34,7 +35,7 @@ EXPORTED_SYMBOLS = [
     "b200ml_where", "b200ml_compare", "b200ml_maxpool2d", "b200ml_wait_probe", "b200ml_strided_copy_parts",
     "b200ml_peer_allgather", "b200ml_ipc_export", "b200ml_ipc_open", "b200ml_ipc_close",
     "b200ml_conv_prepack_bytes", "b200ml_conv_prepack", "b200ml_plan_create", "b200ml_plan_destroy", "b200ml_plan_run",
-    "b200ml_gemm_prepack_bytes", "b200ml_gemm_prepack", "b200ml_gemm_packed",
+    "b200ml_gemm_prepack_bytes", "b200ml_gemm_prepack", "b200ml_gemm_packed", "b200ml_conv_channels_last",
 ]
 
 
@@ -148,6 +149,7 @@ def load_library(path=None):
         lib.b200ml_transpose.argtypes = [vp, c_i32, vp, vp, c_i32, i64p, i32p, vp]
         lib.b200ml_cast.argtypes = [vp, c_i32, c_i32, vp, vp, c_i64, vp]
         lib.b200ml_conv2d.argtypes = [vp, ctypes.POINTER(ConvParams), vp]
+        lib.b200ml_conv_channels_last.argtypes = [vp, ctypes.POINTER(ConvParams)]
         lib.b200ml_conv_prepack_bytes.argtypes = [vp, ctypes.POINTER(ConvParams)]
         lib.b200ml_conv_prepack_bytes.restype = ctypes.c_int64
         lib.b200ml_conv_prepack.argtypes = [vp, ctypes.POINTER(ConvParams), vp, vp]

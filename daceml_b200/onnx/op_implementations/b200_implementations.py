@@ -617,7 +617,7 @@ def _prepacked_conv_weights(node, state, sdfg, x, strides, pads, dil, group, gat
                 t = t.to(dev)
             tensors[conn] = t.contiguous()
     w = tensors["W"]
-    if w.dtype != torch.float32 or not w.is_contiguous():
+    if w.dtype not in FLOAT_TYPES or not w.is_contiguous():
         return None
     return K.conv_prepack(tuple(x.shape), w, bias=tensors.get("B"), strides=strides, pads=pads, dilations=dil, group=group, gate=gate)
 
@@ -692,6 +692,7 @@ class B200FusedConv(ONNXForward):
         x, w = in_desc_with_name(node, state, sdfg, "X"), in_desc_with_name(node, state, sdfg, "W")
         strides, dil, pads, group = _conv_geometry(node, x, w)
         act = _ACT[node.activation]
+        act |= (L.CONV_X_NHWC if x.channels_last else 0) | (L.CONV_Y_NHWC if out_desc_with_name(node, state, sdfg, "Y").channels_last else 0)
         packed = _prepacked_conv_weights(node, state, sdfg, x, strides, pads, dil, group, _has_in(node, state, "Gate"))
 
         def run(ins, outs):

@@ -38,6 +38,8 @@ class Data:
         self.transient = transient
         # name of the array whose storage this one shares (a reshape of it); the counterpart of ``dace.data.View``
         self.view_of = None
+        # an NCHW tensor between two convolutions that keeps its values in channels-last order
+        self.channels_last = False
 
     @property
     def strides(self):

@@ -670,5 +670,35 @@ def alias_reshapes(sdfg, state):
     return count
 
 
+@_each_state
+def keep_channels_last(sdfg, state):
+    """A transient written by one fp16 convolution and read by others only as their X keeps its values channels-last, the
+    order the tensor-core kernel reads (``csrc/conv_f16.cu``): no turn between the two.  Run last, before expansion."""
+    from daceml_b200 import kernels as K
+
+    if not torch.cuda.is_available():
+        return 0
+
+    def takes(cv, **last):
+        x, w = sdfg.arrays[_in(state, cv, "X")], sdfg.arrays[_in(state, cv, "W")]
+        return K.conv_channels_last(x.shape, x.dtype, w.shape, None, strides=cv.strides or (1, 1), pads=cv.pads or (0, 0, 0, 0),
+                                    dilations=cv.dilations or (1, 1), group=int(cv.group or 1), **last)
+
+    count = 0
+    for cv in _nodes(state, "FusedConv"):
+        y = _out(state, cv, "Y")
+        desc, users = sdfg.arrays[y], _consumers(state, y)
+        if (not desc.transient or desc.channels_last or desc.view_of is not None or any(d.view_of == y for d in sdfg.arrays.values())
+                or len(desc.shape) != 4 or _in(state, cv, "Residual") is not None or _out(state, cv, "Pool") is not None or not users):
+            continue
+        if any(type(n) is not donnx.get_onnx_node("FusedConv") or c != "X" or _in(state, n, "Gate") is not None
+               or _out(state, n, "Pool") is not None for n, c in users):
+            continue
+        if takes(cv, y_last=True) and all(takes(n, x_last=True) for n, _ in users):
+            desc.channels_last = True
+            count += 1
+    return count
+
+
 PATTERNS = [remove_identity, fold_batchnorm_into_conv, fuse_gelu, fuse_swish, fuse_layernorm, fuse_linear, fuse_matmul_epilogue, fuse_attention, pack_qkv, fuse_conv,
             fuse_squeeze_excite, fuse_conv_residual]

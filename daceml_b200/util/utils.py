@@ -88,4 +88,7 @@ def auto_optimize(sdfg, cuda=True, simplify=False, fold_constants=True, fuse=Tru
     if views:
         from daceml_b200.transformation.patterns import alias_reshapes
         alias_reshapes(sdfg)
+    if fuse:
+        from daceml_b200.transformation.patterns import keep_channels_last
+        keep_channels_last(sdfg)
     expand_onnx_nodes(sdfg)

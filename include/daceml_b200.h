@@ -312,9 +312,15 @@ int b200ml_maxpool2d(b200ml_ctx* ctx, int32_t dtype, const void* x, void* y, int
 /* Convolution and squeeze-excite                                             */
 /* ------------------------------------------------------------------------- */
 
+/* Flags beside the activation in b200ml_conv_params.act: X is / Y is to be written channels-last ([n, h, w, c]; for a tensor
+ * that stays between two convolutions).  fp16, group 1, channels a multiple of 8, 16-byte aligned, no gate on X, no pool; a
+ * residual is laid out like Y.  Other convolutions return B200ML_ERR_UNSUPPORTED; b200ml_conv_channels_last tells beforehand
+ * (1: this convolution takes the flags in its act; the tensor pointers are not read). */
+enum { B200ML_CONV_X_NHWC = 256, B200ML_CONV_Y_NHWC = 512 };
+
 typedef struct {
     int32_t dtype; /* B200ML_F32 (B200ML_F16 storage with fp32 accumulate also accepted) */
-    int32_t act;   /* 0, B200ML_EPI_RELU or B200ML_EPI_SWISH applied after bias */
+    int32_t act;   /* 0, B200ML_EPI_RELU or B200ML_EPI_SWISH applied after bias; plus B200ML_CONV_* flags */
     int64_t n, c, h, w;  /* X is [n, c, h, w] */
     int64_t m, kh, kw;   /* W is [m, c / group, kh, kw] */
     int64_t stride_h, stride_w;
@@ -336,7 +342,8 @@ typedef struct {
  * strided, padded and grouped convolutions.  fp32 group-1 convolutions run on the tensor cores at
  * fp32 accuracy (three TF32 products per term): stride-1 1x1 kernels with 8..256 output channels,
  * and kernels up to 7 x 7 with stride 1 or 2 whose reduction has 64 terms or more as an implicit GEMM; both use
- * the context's scratch for the split weights, so calls sharing a context must not overlap. */
+ * the context's scratch for the split weights, so calls sharing a context must not overlap.  fp16 group-1 convolutions run
+ * on the tensor cores over a channels-last copy of X in the same scratch (unless X is channels-last already). */
 int b200ml_conv2d(b200ml_ctx* ctx, const b200ml_conv_params* p, b200ml_stream stream);
 /* Weights that do not change between calls can be prepared once (the role cuDNN's filter descriptors and a framework's
  * weight pre-packing play for the reference's GPU route, cudnn_implementations.py:205-240): the tensor-core kernels
@@ -345,6 +352,7 @@ int b200ml_conv2d(b200ml_ctx* ctx, const b200ml_conv_params* p, b200ml_stream st
  * tensor pointers are not read), 0 if the convolution runs on a kernel that takes the weights as they are.
  * b200ml_conv_prepack writes it (16-byte aligned device memory of that size, owned by the caller); later calls pass it
  * as p->packed_weight together with the same weight, bias, shapes and attributes. */
+int32_t b200ml_conv_channels_last(b200ml_ctx* ctx, const b200ml_conv_params* p);
 int64_t b200ml_conv_prepack_bytes(b200ml_ctx* ctx, const b200ml_conv_params* p);
 int b200ml_conv_prepack(b200ml_ctx* ctx, const b200ml_conv_params* p, void* packed, b200ml_stream stream);
 
