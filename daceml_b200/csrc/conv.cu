@@ -13,10 +13,10 @@ namespace b200ml {
 
 int reduce(const b200ml_ctx* ctx, int dtype, int op, const void* x, void* y, int64_t outer, int64_t red, int64_t inner,
            cudaStream_t s);
-bool conv_f16_applies(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow);
-int64_t conv_f16_pack_bytes(const b200ml_conv_params* p);
-int conv_f16_pack(const b200ml_ctx* ctx, const b200ml_conv_params* p, void* packed, cudaStream_t s);
-int conv_f16(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow, cudaStream_t s);
+bool conv_nhwc_applies(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow);
+int64_t conv_nhwc_pack_bytes(const b200ml_conv_params* p);
+int conv_nhwc_pack(const b200ml_ctx* ctx, const b200ml_conv_params* p, void* packed, cudaStream_t s);
+int conv_nhwc(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow, cudaStream_t s);
 bool conv1x1_tensor_core_applies(const b200ml_ctx* ctx, const b200ml_conv_params* p);
 int conv1x1_tensor_core(const b200ml_ctx* ctx, const b200ml_conv_params* p, cudaStream_t stream);
 bool conv_igemm_applies(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow);
@@ -598,9 +598,10 @@ static int conv2d_fast(const b200ml_ctx* ctx, const b200ml_conv_params* p, const
                        bool* pooled) {
     *launched = false;
     *pooled = false;
-    if (conv_f16_applies(ctx, p, g.oh, g.ow)) {  // fp16, group 1: implicit GEMM on the tensor core over channels-last operands
+    const bool nhwc = conv_nhwc_applies(ctx, p, g.oh, g.ow);
+    if (p->dtype == B200ML_F16 && nhwc) {  // fp16, group 1: implicit GEMM on the tensor core over channels-last operands
         *launched = true;
-        return conv_f16(ctx, p, g.oh, g.ow, s);
+        return conv_nhwc(ctx, p, g.oh, g.ow, s);
     }
     if (p->act & (B200ML_CONV_X_NHWC | B200ML_CONV_Y_NHWC))
         return fail(B200ML_ERR_UNSUPPORTED, "conv: channels-last tensors need a convolution the fp16 tensor-core kernel takes");
@@ -609,6 +610,10 @@ static int conv2d_fast(const b200ml_ctx* ctx, const b200ml_conv_params* p, const
     if (conv1x1_tensor_core_applies(ctx, p)) {  // 1x1, stride 1: the tensor-core kernel (3 x TF32), HBM-bound
         *launched = true;
         return conv1x1_tensor_core(ctx, p, s);
+    }
+    if (nhwc && !conv_igemm_applies(ctx, p, g.oh, g.ow)) {  // fp32 on channels-last copies of X (3 x TF32)
+        *launched = true;
+        return conv_nhwc(ctx, p, g.oh, g.ow, s);
     }
     if (conv_igemm_applies(ctx, p, g.oh, g.ow)) {  // k x k, stride 1, group 1: implicit GEMM on the tensor core (3 x TF32)
         *launched = true;
@@ -699,8 +704,8 @@ int conv2d(const b200ml_ctx* ctx, const b200ml_conv_params* p, cudaStream_t s) {
     return B200ML_OK;
 }
 
-// Which tensor-core kernel (if any) takes this convolution: 1 = the 1x1 kernel, 2 = the fp32 implicit GEMM, 3 = the fp16 one,
-// 0 = none.
+// Which tensor-core kernel (if any) takes this convolution: 1 = the 1x1 kernel, 2 = the implicit GEMM over NCHW,
+// 3 = the one over channels-last operands, 0 = none.
 static int conv_tensor_core_kind(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t* ow_out) {
     if (p->group < 1 || p->stride_h < 1 || p->stride_w < 1 || p->dil_h < 1 || p->dil_w < 1 || p->kh < 1 || p->kw < 1) return 0;
     const int64_t eh = p->h + p->pad_top + p->pad_bottom - p->dil_h * (p->kh - 1) - 1;
@@ -712,9 +717,10 @@ static int conv_tensor_core_kind(const b200ml_ctx* ctx, const b200ml_conv_params
     b200ml_conv_params q = *p;
     if (!q.x) q.x = reinterpret_cast<const void*>(uintptr_t(256));
     if (!q.y) q.y = reinterpret_cast<void*>(uintptr_t(256));
-    if (conv_f16_applies(ctx, &q, oh, ow)) return 3;
+    if (q.dtype == B200ML_F16) return conv_nhwc_applies(ctx, &q, oh, ow) ? 3 : 0;
     if (conv1x1_tensor_core_applies(ctx, &q)) return 1;
     if (conv_igemm_applies(ctx, &q, oh, ow)) return 2;
+    if (conv_nhwc_applies(ctx, &q, oh, ow)) return 3;
     return 0;
 }
 
@@ -727,7 +733,7 @@ int32_t conv_channels_last(const b200ml_ctx* ctx, const b200ml_conv_params* p) {
 int64_t conv_prepack_bytes(const b200ml_ctx* ctx, const b200ml_conv_params* p) {
     int64_t ow = 0;
     const int kind = conv_tensor_core_kind(ctx, p, &ow);
-    return kind == 3 ? conv_f16_pack_bytes(p) : kind == 1 ? conv1x1_pack_bytes(p) : (kind == 2 ? conv_igemm_pack_bytes(p, ow) : 0);
+    return kind == 3 ? conv_nhwc_pack_bytes(p) : kind == 1 ? conv1x1_pack_bytes(p) : (kind == 2 ? conv_igemm_pack_bytes(p, ow) : 0);
 }
 
 int conv_prepack(const b200ml_ctx* ctx, const b200ml_conv_params* p, void* packed, cudaStream_t s) {
@@ -735,7 +741,7 @@ int conv_prepack(const b200ml_ctx* ctx, const b200ml_conv_params* p, void* packe
     const int kind = conv_tensor_core_kind(ctx, p, &ow);
     B200ML_REQUIRE(kind != 0, "conv_prepack: this convolution takes its weights as they are (b200ml_conv_prepack_bytes returns 0)");
     B200ML_REQUIRE(packed && aligned16(packed) && p->weight, "conv_prepack: the packed buffer must be 16-byte aligned device memory, the weights given");
-    return kind == 3 ? conv_f16_pack(ctx, p, packed, s) : kind == 1 ? conv1x1_pack(ctx, p, packed, s) : conv_igemm_pack(ctx, p, ow, packed, s);
+    return kind == 3 ? conv_nhwc_pack(ctx, p, packed, s) : kind == 1 ? conv1x1_pack(ctx, p, packed, s) : conv_igemm_pack(ctx, p, ow, packed, s);
 }
 
 int se_gate(const b200ml_ctx*, int dtype, const void* pooled, const void* w1, const void* b1, const void* w2,

@@ -1,0 +1,643 @@
+// Convolution (group 1; any kernel, stride up to 8, dilation, padding; fp16 or fp32) as an implicit GEMM on tcgen05:
+//     Y[n, m, h, w] = act(B[m] + sum_{c, i, j} W[m, c, i, j] * X[n, c, sh h - pad_top + dh i, sw w - pad_left + dw j] * gate[n, c]) + R[n, m, h, w]
+// (the reference's routes: daceml/onnx/op_implementations/img_op_implementations.py:217-288, cudnn_implementations.py:123-410).
+//
+// X is read channels-last ([N][H][W][Cp], rows of Cp channels padded to 16 bytes): a box of {one 128-byte chunk of channels,
+// wb x hb pixels, nb images} at the window position of one kernel tap is then a K-major operand tile that the TMA unit lays
+// out by itself - the padding is its zero fill, a stride its element stride - so there is no im2col buffer and no shifting by
+// warps.  An NCHW X is turned by a small kernel first (conv_prepare_kernel, which also applies a squeeze-excite gate); between
+// two fp16 convolutions of a graph the epilogue writes channels-last directly (B200ML_CONV_X_NHWC / Y_NHWC) and the turn is
+// not needed.  The reduction runs over (tap, chunk of 32, 64 or 128 bytes of channels); the weights of a step come as one
+// bulk copy from a copy laid out beforehand in the operand tile's swizzled order (once per constant weight, else by the
+// turn's launch).
+// fp32 runs as 3 x TF32 (kind::tf32; see gemm_f32.cu for the split and the four accumulators): the turn writes a hi and a lo
+// copy of X, the weights carry both parts, a step loads four tiles.
+//
+// One 128-pixel x BN-channel tile per CTA, two to four CTAs per SM so that one's epilogue runs under the others' main loops; few
+// tiles split the reduction over a cluster (partial tiles through distributed shared memory, summed in rank order).
+// The box wb x hb x nb <= 128 is chosen to cover the output with the fewest tiles (56 x 56: 28 x 4).
+// Bound: L2 -> shared memory traffic (every tap re-reads its window) and, on small layers, latency.
+//
+// Measured (us, direct FMA kernel before -> turn + convolution), fp16: two 3x3, 64 -> 64 at 56 x 56, 8 images 535 -> 16.5 (one
+// turn); 3x3 32 -> 36 at 117 x 117, 24 images 17.5 + 46; 1x1 24 -> 144 at 56 x 56, 32 images 8.8 + 42.
+// fp32, where the kernels that read NCHW do not apply (conv1x1_tc.cu, conv_igemm.cu: large outputs): 3x3 64 -> 64 at 56 x 56,
+// one image 235 -> 13.4; 256 -> 256 at 14 x 14, 8 images 954 -> 33.5; 7x7 stride 2, 3 -> 64 at 150 x 150, 4 images 96.7 -> 37.
+#include "gemm_common.cuh"
+#include "conv_tc.cuh"
+
+namespace b200ml {
+
+namespace {
+
+constexpr int H_BM = 128;
+constexpr int H_THREADS = 64 + 128;         // TMA warp, MMA warp, four epilogue warps
+constexpr int H_PIPE_BYTES = 96 * 1024;     // operand stages of a CTA: two CTAs fit on an SM ...
+constexpr int H_MAX_STAGES = 8;
+constexpr int H_PART_LD = H_BM + 4;         // floats between columns of a parked partial tile
+constexpr int H_PACK_ROWS = 32;
+
+template <typename T>
+struct HType {
+    static constexpr int PARTS = sizeof(T) == 4 ? 2 : 1;  // operand parts: hi and lo of fp32
+    static constexpr int NACC = sizeof(T) == 4 ? 4 : 1;   // accumulators the steps are dealt to
+    static constexpr int EPC = 16 / sizeof(T);            // elements of a 16-byte unit
+    // ... and up to four (fp16) where the reduction is short; never more than the tensor memory of an SM serves
+    static constexpr int MIN_PIPE_BYTES = sizeof(T) == 4 ? 80 * 1024 : 48 * 1024;
+};
+
+template <typename T>
+struct ConvHArgs {
+    const T* w;              // packed weights: [step][part][row (padded)][chunk], swizzled
+    const T* bias;
+    const T* residual;
+    T* y;
+    int32_t n, m, oh, ow;
+    int32_t wb, hb, nb;                       // pixels of a tile
+    int32_t tiles_w, tiles_h, tiles_n, tiles_m;
+    int32_t kcb, chunks, steps, kw;           // bytes of channels per step, chunks per tap, steps in all
+    int32_t packed_rows, stages, pipe_bytes, split;
+    int32_t sh, sw, dh, dw, pad_top, pad_left;
+    int32_t act, y_nhwc;
+    int32_t* status;
+};
+
+__device__ __forceinline__ float h_load(const float* p) { return __ldg(p); }
+__device__ __forceinline__ float h_load(const __half* p) { return __half2float(__ldg(p)); }
+__device__ __forceinline__ void h_store(float* p, float v) { *p = v; }
+__device__ __forceinline__ void h_store(__half* p, float v) { *p = __float2half_rn(v); }
+
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(ptx::smem_u32(bar))
+                 : "memory");
+}
+
+// K-major operand tile with rows of kcb bytes in the matching swizzle (128, 64 or 32 bytes): 8-row groups are 8 * kcb bytes
+// apart.
+__device__ __forceinline__ uint64_t conv_desc(uint32_t addr, int kcb) {
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((addr & 0x3ffffu) >> 4);
+    d |= 1ull << 16;
+    d |= static_cast<uint64_t>((kcb >> 1) & 0x3fff) << 32;  // (8 * kcb) >> 4
+    d |= 1ull << 46;
+    d |= static_cast<uint64_t>(kcb == 128 ? 2 : (kcb == 64 ? 4 : 6)) << 61;
+    return d;
+}
+
+// Sixteen channels from m0 on of one output pixel.
+template <typename T>
+__device__ __forceinline__ void finish16(const ConvHArgs<T>& g, float (&v)[16], int m0, int64_t pix_nchw, int64_t pix_nhwc) {
+    const int64_t plane = static_cast<int64_t>(g.oh) * g.ow;
+    if (g.bias) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (m0 + j < g.m) v[j] += h_load(g.bias + m0 + j);
+    }
+    if (g.act) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = conv_act(v[j], g.act);
+    }
+    if constexpr (sizeof(T) == 2) {
+        if (g.y_nhwc) {  // m is a multiple of 8 here
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (m0 + 8 * u < g.m) {
+                    float o[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) o[j] = v[8 * u + j];
+                    if (g.residual) {
+                        float q[8];
+                        unpack8(__ldg(reinterpret_cast<const uint4*>(g.residual + pix_nhwc + m0 + 8 * u)), q);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) o[j] += q[j];
+                    }
+                    *reinterpret_cast<uint4*>(g.y + pix_nhwc + m0 + 8 * u) = pack8(o);
+                }
+            }
+            return;
+        }
+    }
+    if (g.residual) {
+        float r[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) r[j] = m0 + j < g.m ? h_load(g.residual + pix_nchw + (m0 + j) * plane) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] += r[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if (m0 + j < g.m) h_store(g.y + pix_nchw + (m0 + j) * plane, v[j]);
+}
+
+template <typename T, int BN>
+__global__ void __launch_bounds__(H_THREADS, sizeof(T) == 4 ? 2 : 4)
+conv_nhwc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_xl, const ConvHArgs<T> g) {
+    constexpr int PARTS = HType<T>::PARTS, NACC = HType<T>::NACC;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + g.pipe_bytes);
+    uint64_t* empty_bar = full_bar + H_MAX_STAGES;
+    uint64_t* acc_bar = empty_bar + H_MAX_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = g.split > 1 ? static_cast<int>(ptx::cluster_ctarank()) : 0;
+    int t = blockIdx.x / g.split;
+    const int mt = t % g.tiles_m;  // the channel blocks of one window run at the same time: its second read hits L2
+    t /= g.tiles_m;
+    const int w0 = (t % g.tiles_w) * g.wb;
+    t /= g.tiles_w;
+    const int h0 = (t % g.tiles_h) * g.hb;
+    const int n0 = (t / g.tiles_h) * g.nb;
+    const int per = (g.steps + g.split - 1) / g.split;
+    const int begin = rank * per < g.steps ? rank * per : g.steps;
+    const int nk = (begin + per < g.steps ? begin + per : g.steps) - begin;
+    const int a_bytes = H_BM * g.kcb, b_bytes = BN * g.kcb, stage_bytes = PARTS * (a_bytes + b_bytes);
+
+    if (warp == 0 && lane == 0) ptx::prefetch_tensormap(&tmap_x);
+    if (warp == 1) {
+        if (lane == 0) {
+            for (int s = 0; s < g.stages; ++s) {
+                ptx::mbar_init(&full_bar[s], 1);
+                ptx::mbar_init(&empty_bar[s], 1);
+            }
+            ptx::mbar_init(acc_bar, 1);
+            ptx::fence_mbar_init();
+        }
+        __syncwarp();
+        ptx::tmem_alloc(tmem_slot, NACC * BN);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    pdl_launch_dependents();  // after the allocation: an early CTA of the next kernel cannot take this CTA's tensor memory
+    ptx::tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        // ------------------------------ producer: a box of X and a block of weights per step and part ------------------------------
+        if (ptx::elect_one()) {
+            pdl_wait();
+            const int rows = g.packed_rows - mt * BN < BN ? g.packed_rows - mt * BN : BN;
+            const uint32_t w_bytes = rows * g.kcb, x_bytes = g.wb * g.hb * g.nb * g.kcb;
+            const int kc = g.kcb / static_cast<int>(sizeof(T));
+            int stage = 0;
+            uint32_t phase = 0;
+            int chunk = begin % g.chunks, tap = begin / g.chunks;
+            int ti = tap / g.kw, tj = tap - ti * g.kw;
+            for (int i = 0; i < nk; ++i) {
+                if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
+                    atomicExch(g.status, DEV_TIMEOUT_PRODUCER);
+                    break;
+                }
+                uint8_t* dst = smem + stage * stage_bytes;
+                ptx::mbar_expect_tx(&full_bar[stage], PARTS * (w_bytes + x_bytes));
+                const T* w = g.w + (static_cast<int64_t>(begin + i) * PARTS * g.packed_rows + mt * BN) * kc;
+                const int x0 = w0 * g.sw - g.pad_left + tj * g.dw, y0 = h0 * g.sh - g.pad_top + ti * g.dh;
+                bulk_copy(ptx::smem_u32(dst + PARTS * a_bytes), w, w_bytes, &full_bar[stage]);
+                ptx::tma_load_4d(dst, &tmap_x, &full_bar[stage], chunk * kc, x0, y0, n0);
+                if (PARTS == 2) {
+                    bulk_copy(ptx::smem_u32(dst + PARTS * a_bytes + b_bytes), w + static_cast<int64_t>(g.packed_rows) * kc, w_bytes, &full_bar[stage]);
+                    ptx::tma_load_4d(dst + a_bytes, &tmap_xl, &full_bar[stage], chunk * kc, x0, y0, n0);
+                }
+                if (++chunk == g.chunks) {
+                    chunk = 0;
+                    if (++tj == g.kw) tj = 0, ++ti;
+                }
+                if (++stage == g.stages) stage = 0, phase ^= 1;
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // ------------------------------ MMA issuer ------------------------------
+        if (ptx::elect_one()) {
+            // fp32 accumulator, M = 128, N = BN, both operands K-major: fp16, or tf32 (format 2)
+            constexpr uint32_t idesc = ptx::make_idesc_f16(H_BM, BN, 0, 0) | (PARTS == 2 ? (2u << 7) | (2u << 10) : 0u);
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int i = 0; i < nk; ++i) {
+                if (!ptx::mbar_wait(&full_bar[stage], phase)) {
+                    atomicExch(g.status, DEV_TIMEOUT_MMA);
+                    ok = false;
+                    break;
+                }
+                ptx::tc_fence_after();
+                const uint32_t a = ptx::smem_u32(smem + stage * stage_bytes);
+                const uint32_t d = tmem_base + (i % NACC) * BN;
+                const uint64_t da = conv_desc(a, g.kcb), db = conv_desc(a + PARTS * a_bytes, g.kcb);
+                const uint64_t dal = conv_desc(a + a_bytes, g.kcb), dbl = conv_desc(a + PARTS * a_bytes + b_bytes, g.kcb);
+                for (int kk = 0; kk < g.kcb / 32; ++kk) {  // 32 bytes along the line per step
+                    const uint32_t acc = (i >= NACC || kk != 0) ? 1u : 0u;
+                    if constexpr (PARTS == 2) {  // the two small terms first, the large one last
+                        convtc::pw_mma(d, dal + 2 * kk, db + 2 * kk, idesc, acc);
+                        convtc::pw_mma(d, da + 2 * kk, dbl + 2 * kk, idesc, 1u);
+                        convtc::pw_mma(d, da + 2 * kk, db + 2 * kk, idesc, 1u);
+                    } else {
+                        ptx::mma_f16_ss(d, da + 2 * kk, db + 2 * kk, idesc, acc);
+                    }
+                }
+                ptx::mma_commit(&empty_bar[stage]);
+                if (++stage == g.stages) stage = 0, phase ^= 1;
+            }
+            if (ok && nk > 0) ptx::mma_commit(acc_bar);
+        }
+        __syncwarp();
+    }
+    // ------------------------------ epilogue: a lane = a pixel, a warp = 32 pixels ------------------------------
+    const int quarter = warp & 3;
+    const int row = quarter * 32 + lane;
+    const int pw = w0 + row % g.wb, ph = h0 + (row / g.wb) % g.hb, pn = n0 + row / (g.wb * g.hb);
+    const bool pix_ok = row < g.wb * g.hb * g.nb && pw < g.ow && ph < g.oh && pn < g.n;
+    const int64_t pix_nchw = (static_cast<int64_t>(pn) * g.m * g.oh + ph) * g.ow + pw;
+    const int64_t pix_nhwc = ((static_cast<int64_t>(pn) * g.oh + ph) * g.ow + pw) * g.m;
+    float* partial = reinterpret_cast<float*>(smem);
+    if (warp >= 2) {
+        bool ok = true;
+        pdl_wait();  // the residual, and Y itself, may be a predecessor's
+        if (nk > 0 && !ptx::mbar_wait(acc_bar, 0)) {
+            if (lane == 0) atomicExch(g.status, DEV_TIMEOUT_EPILOGUE);
+            ok = false;
+        }
+        __syncwarp();
+        ptx::tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; ok && c < BN; c += 16) {
+            if (mt * BN + c >= g.m) break;  // warp-uniform
+            float v[16];
+            if (nk > 0) {
+                uint32_t r[NACC][16];
+                const int nacc = nk < NACC ? nk : NACC;
+#pragma unroll
+                for (int q = 0; q < NACC; ++q)
+                    if (q < nacc) ptx::tmem_ld_32x32b_x16(tmem_base + q * BN + c + (static_cast<uint32_t>(quarter * 32) << 16), r[q]);
+                ptx::tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[0][j]);
+#pragma unroll
+                for (int q = 1; q < NACC; ++q)
+                    if (q < nacc) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[q][j]);
+                    }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = 0.0f;
+            }
+            if (g.split == 1) {
+                if (pix_ok) finish16(g, v, mt * BN + c, pix_nchw, pix_nhwc);
+                __syncwarp();
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) partial[(c + j) * H_PART_LD + row] = v[j];
+            }
+        }
+        ptx::tc_fence_before();
+    }
+    if (g.split > 1) {
+        ptx::cluster_sync_acq_rel();
+        if (warp >= 2) {
+            // this CTA's share of the channels, in pieces of sixteen
+            const int share = BN / g.split;  // 16 or more
+            for (int c = rank * share; c < (rank + 1) * share; c += 16) {
+                if (mt * BN + c >= g.m) break;
+                float v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = 0.0f;
+                for (int q = 0; q < g.split; ++q) {  // rank order: the same sum on every run
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] += ptx::ld_shared_cluster_f32(partial + (c + j) * H_PART_LD + row, q);
+                }
+                if (pix_ok) finish16(g, v, mt * BN + c, pix_nchw, pix_nhwc);
+            }
+        }
+        ptx::cluster_sync_acq_rel();  // no CTA leaves while a peer may still read its partial tile
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        ptx::tc_fence_after();
+        if (*reinterpret_cast<volatile int32_t*>(g.status) != DEV_OK) {
+            for (int i = 0; i < 200; ++i) __nanosleep(1000);  // a wait gave up: let copies and MMAs in flight land
+        }
+        ptx::tmem_dealloc(tmem_base, NACC * BN);
+    }
+}
+
+// What a convolution needs before its main kernel, in one launch: the first `turn_blocks` blocks turn X channels-last
+// ([N][C][HW] -> [N][HW][Cp], zeros in the channels past C, optionally times gate[n][c]; fp32 as a hi and a lo copy), the
+// others lay the weights out ([M][C][kh][kw] -> [tap][chunk][part][row (padded)][chunk] in the operand tile's swizzle).
+// A turning block takes 64 pixels x 128 bytes of channels through shared memory: rows of pixels in, 16-byte units of channels
+// out.  Bound: memory (one read, one or two writes).
+template <typename T>
+struct PrepareArgs {
+    const T* x;
+    const T* gate;
+    T* out;      // hi copy; the lo copy follows `lo_offset` elements later
+    int64_t lo_offset;
+    int32_t c, cp, hw, vec, p_tiles, c_tiles;
+    int64_t turn_blocks;
+    const T* w;
+    T* w_out;
+    int32_t m, taps, kc, chunks, rows;
+    int64_t units;
+};
+
+// hi = the value rounded to nearest-even at 10 mantissa bits (TF32), lo = value - hi; infinities and NaNs stay in hi.
+__device__ __forceinline__ void h_split(float x, float& hi, float& lo) {
+    const uint32_t b = __float_as_uint(x);
+    const bool finite = (b & 0x7f800000u) != 0x7f800000u;
+    hi = __uint_as_float(finite ? ((b + 0xfffu + ((b >> 13) & 1u)) & 0xffffe000u) : b);
+    lo = finite ? x - hi : 0.0f;
+}
+
+// A 16-byte unit of EPC values; of fp32 values its hi part to `dst` and its lo part to `dst + lo_offset`.
+__device__ __forceinline__ void store_unit(__half* dst, int64_t, const float (&v)[8]) { *reinterpret_cast<uint4*>(dst) = pack8(v); }
+__device__ __forceinline__ void store_unit(float* dst, int64_t lo_offset, const float (&v)[4]) {
+    float4 hi, lo;
+    h_split(v[0], hi.x, lo.x), h_split(v[1], hi.y, lo.y), h_split(v[2], hi.z, lo.z), h_split(v[3], hi.w, lo.w);
+    *reinterpret_cast<float4*>(dst) = hi;
+    *reinterpret_cast<float4*>(dst + lo_offset) = lo;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) conv_prepare_kernel(const PrepareArgs<T> g) {
+    constexpr int EPC = HType<T>::EPC, CH = 8 * EPC;  // channels of a turning block
+    constexpr int LD = sizeof(T) == 2 ? 66 : 65;      // odd numbers of 32-bit words between channels
+    __shared__ T tile[CH][LD];
+    pdl_launch_dependents();
+    pdl_wait();
+    if (static_cast<int64_t>(blockIdx.x) < g.turn_blocks) {
+        const int p0 = (blockIdx.x % g.p_tiles) * 64, c0 = (blockIdx.x / g.p_tiles % g.c_tiles) * CH;
+        const int64_t img = blockIdx.x / g.p_tiles / g.c_tiles;
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int p = p0 + lane * 2;
+#pragma unroll
+        for (int i = 0; i < EPC; ++i) {
+            const int ch = c0 + warp + 8 * i;
+            float a = 0.0f, b = 0.0f;
+            if (ch < g.c) {
+                const T* src = g.x + (img * g.c + ch) * g.hw + p;
+                if (g.vec && p + 1 < g.hw) {
+                    if constexpr (sizeof(T) == 2) {
+                        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(src));
+                        a = v.x, b = v.y;
+                    } else {
+                        const float2 v = __ldg(reinterpret_cast<const float2*>(src));
+                        a = v.x, b = v.y;
+                    }
+                } else {
+                    if (p < g.hw) a = h_load(src);
+                    if (p + 1 < g.hw) b = h_load(src + 1);
+                }
+                if (g.gate) {
+                    const float gv = h_load(g.gate + img * g.c + ch);
+                    a *= gv, b *= gv;
+                }
+            }
+            h_store(&tile[warp + 8 * i][lane * 2], a);
+            h_store(&tile[warp + 8 * i][lane * 2 + 1], b);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int unit = threadIdx.x + 256 * i, cg = unit & 7, px = unit >> 3;
+            if (c0 + cg * EPC < g.cp && p0 + px < g.hw) {
+                float o[EPC];
+#pragma unroll
+                for (int j = 0; j < EPC; ++j) o[j] = static_cast<float>(tile[cg * EPC + j][px]);
+                store_unit(g.out + (img * g.hw + p0 + px) * g.cp + c0 + cg * EPC, g.lo_offset, o);
+            }
+        }
+        return;
+    }
+    const int64_t block = blockIdx.x - g.turn_blocks, blocks = gridDim.x - g.turn_blocks;
+    const int parts = HType<T>::PARTS, per_row = g.kc / EPC;
+    for (int64_t i = block * blockDim.x + threadIdx.x; i < g.units; i += blocks * blockDim.x) {
+        const int u = static_cast<int>(i % per_row);
+        int64_t rest = i / per_row;
+        const int row = static_cast<int>(rest % g.rows);
+        rest /= g.rows;
+        const int chunk = static_cast<int>(rest % g.chunks), tap = static_cast<int>(rest / g.chunks);
+        float o[EPC];
+#pragma unroll
+        for (int j = 0; j < EPC; ++j) {
+            const int ch = chunk * g.kc + u * EPC + j;
+            o[j] = row < g.m && ch < g.c ? h_load(g.w + (static_cast<int64_t>(row) * g.c + ch) * g.taps + tap) : 0.0f;
+        }
+        const int sw = per_row == 8 ? (u ^ (row & 7)) : (per_row == 4 ? (u ^ ((row >> 1) & 3)) : (u ^ ((row >> 2) & 1)));
+        store_unit(g.w_out + (static_cast<int64_t>(tap * g.chunks + chunk) * parts * g.rows + row) * g.kc + sw * EPC,
+                   static_cast<int64_t>(g.rows) * g.kc, o);
+    }
+}
+
+// Channels rounded up to 16-byte rows, and the channels of a reduction step: 128, 64 or 32 bytes.
+template <typename T>
+int64_t padded_channels(int64_t c) { return ceil_div(c, HType<T>::EPC) * HType<T>::EPC; }
+template <typename T>
+int step_channels(int64_t cp) {
+    const int64_t bytes = cp * (int64_t)sizeof(T);
+    return (bytes > 64 ? 128 : (bytes > 32 ? 64 : 32)) / (int)sizeof(T);
+}
+int64_t padded_rows(int64_t m) { return ceil_div(m, H_PACK_ROWS) * H_PACK_ROWS; }
+
+template <typename T>
+int64_t pack_elements(const b200ml_conv_params* p) {
+    const int64_t cp = padded_channels<T>(p->c);
+    const int kc = step_channels<T>(cp);
+    return p->kh * p->kw * ceil_div(cp, kc) * HType<T>::PARTS * padded_rows(p->m) * kc;
+}
+
+template <typename T>
+int launch_prepare(const b200ml_ctx* ctx, PrepareArgs<T>& a, const b200ml_conv_params* p, T* w_out, cudaStream_t s) {
+    int64_t pack_blocks = 0;
+    if (w_out) {
+        const int64_t cp = padded_channels<T>(p->c);
+        a.w = static_cast<const T*>(p->weight), a.w_out = w_out;
+        a.c = (int32_t)p->c, a.m = (int32_t)p->m, a.taps = (int32_t)(p->kh * p->kw), a.kc = step_channels<T>(cp);
+        a.chunks = (int32_t)ceil_div(cp, a.kc), a.rows = (int32_t)padded_rows(p->m);
+        a.units = (int64_t)a.taps * a.chunks * a.rows * (a.kc / HType<T>::EPC);
+        pack_blocks = ceil_div(a.units, 256);
+        if (pack_blocks > ctx->sm_count * 8) pack_blocks = ctx->sm_count * 8;
+    }
+    B200ML_REQUIRE(a.turn_blocks + pack_blocks < (1ll << 31), "conv: too many blocks");
+    B200ML_CUDA(launch_pdl(conv_prepare_kernel<T>, dim3((unsigned)(a.turn_blocks + pack_blocks)), dim3(256), 0, s, a));
+    return check_launch("conv_prepare");
+}
+
+template <typename T, int BN>
+int launch_conv(const b200ml_ctx* ctx, const CUtensorMap& tx, const CUtensorMap& txl, ConvHArgs<T>& g, cudaStream_t s) {
+    auto kernel = conv_nhwc_kernel<T, BN>;
+    static bool configured[64] = {};  // per instantiation and device
+    if (!configured[ctx->device & 63]) {
+        B200ML_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, H_PIPE_BYTES + 1280));
+        configured[ctx->device & 63] = true;
+    }
+    g.tiles_m = (int32_t)ceil_div(g.m, BN);
+    const int64_t tiles = (int64_t)g.tiles_w * g.tiles_h * g.tiles_n * g.tiles_m;
+    B200ML_REQUIRE(tiles < (1ll << 27), "conv: too many tiles");
+    const int stage_bytes = HType<T>::PARTS * (H_BM + BN) * g.kcb;
+    g.stages = H_PIPE_BYTES / stage_bytes < H_MAX_STAGES ? H_PIPE_BYTES / stage_bytes : H_MAX_STAGES;
+    // Few tiles: the reduction is split while that adds CTAs, every CTA keeps four steps and a share of sixteen channels.
+    g.split = 1;
+    while (g.split < 4 && tiles * g.split * 2 <= ctx->sm_count && g.steps >= g.split * 8 && BN / (g.split * 2) >= 16) g.split *= 2;
+    const int per = (int)ceil_div(g.steps, g.split);
+    if (g.stages > per) g.stages = per;
+    int pipe = g.stages * stage_bytes;
+    if (pipe < HType<T>::MIN_PIPE_BYTES) pipe = HType<T>::MIN_PIPE_BYTES;
+    if (g.split > 1 && pipe < BN * H_PART_LD * 4) pipe = (BN * H_PART_LD * 4 + 1023) & ~1023;
+    g.pipe_bytes = pipe;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * g.split));
+    cfg.blockDim = dim3(H_THREADS);
+    cfg.dynamicSmemBytes = pipe + 1280;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = g.split, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    B200ML_CUDA(cudaLaunchKernelEx(&cfg, kernel, tx, txl, g));
+    return check_launch("conv_nhwc");
+}
+
+template <typename T>
+int conv_impl(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow, cudaStream_t s) {
+    constexpr int PARTS = HType<T>::PARTS;
+    const int64_t cp = padded_channels<T>(p->c);
+    const bool x_nhwc = (p->act & B200ML_CONV_X_NHWC) != 0, y_nhwc = (p->act & B200ML_CONV_Y_NHWC) != 0;
+    B200ML_REQUIRE(!(x_nhwc || y_nhwc) || (!p->pool_sum && sizeof(T) == 2), "conv: channels-last tensors are fp16 and have no pooled output");
+    B200ML_REQUIRE(!x_nhwc || (p->c % 8 == 0 && !p->gate), "conv: a channels-last X needs a multiple of 8 channels and no gate");
+    B200ML_REQUIRE(!y_nhwc || p->m % 8 == 0, "conv: a channels-last Y needs a multiple of 8 channels");
+    char* ws = static_cast<char*>(ctx->workspace);
+    int64_t room = ctx->workspace_bytes;
+    const T* w = static_cast<const T*>(p->packed_weight);
+    T* w_out = nullptr;
+    if (!w) {
+        const int64_t bytes = ceil_div(pack_elements<T>(p) * (int64_t)sizeof(T), 1024) * 1024;
+        if (bytes > room / 2) return fail(B200ML_ERR_WORKSPACE, "conv: the weights (%lld bytes laid out) exceed the workspace", (long long)bytes);
+        w_out = reinterpret_cast<T*>(ws);
+        w = w_out;
+        ws += bytes, room -= bytes;
+    }
+    // images in pieces whose channels-last copy fits the workspace
+    const int64_t image = cp * p->h * p->w;
+    int64_t piece = p->n;
+    if (!x_nhwc) {
+        const int64_t fit = room / (image * PARTS * (int64_t)sizeof(T));
+        if (fit < 1) return fail(B200ML_ERR_WORKSPACE, "conv: an image does not fit the workspace");
+        if (fit < piece) piece = fit;
+        piece = ceil_div(p->n, ceil_div(p->n, piece));
+    }
+    for (int64_t n0 = 0; n0 < p->n; n0 += piece) {
+        const int64_t n = p->n - n0 < piece ? p->n - n0 : piece;
+        const T* x = static_cast<const T*>(p->x) + n0 * p->c * p->h * p->w;
+        PrepareArgs<T> a{};
+        if (!x_nhwc) {
+            a.x = x, a.gate = p->gate ? static_cast<const T*>(p->gate) + n0 * p->c : nullptr;
+            a.out = reinterpret_cast<T*>(ws), a.lo_offset = n * image;
+            a.c = (int32_t)p->c, a.cp = (int32_t)cp, a.hw = (int32_t)(p->h * p->w);
+            a.vec = a.hw % 2 == 0 && reinterpret_cast<uintptr_t>(x) % (2 * sizeof(T)) == 0 ? 1 : 0;
+            a.p_tiles = (int32_t)ceil_div(a.hw, 64), a.c_tiles = (int32_t)ceil_div(cp, 8 * HType<T>::EPC);
+            a.turn_blocks = (int64_t)a.p_tiles * a.c_tiles * n;
+            x = a.out;
+        }
+        if (!x_nhwc || (w_out && n0 == 0)) {
+            const int rc = launch_prepare<T>(ctx, a, p, n0 == 0 ? w_out : nullptr, s);
+            if (rc) return rc;
+        }
+        ConvHArgs<T> g{};
+        g.w = w;
+        g.bias = static_cast<const T*>(p->bias);
+        g.residual = p->residual ? static_cast<const T*>(p->residual) + n0 * p->m * oh * ow : nullptr;
+        g.y = static_cast<T*>(p->y) + n0 * p->m * oh * ow;
+        g.n = (int32_t)n, g.m = (int32_t)p->m, g.oh = (int32_t)oh, g.ow = (int32_t)ow;
+        const int kc = step_channels<T>(cp);
+        g.kcb = kc * (int)sizeof(T), g.chunks = (int32_t)ceil_div(cp, kc);
+        g.steps = (int32_t)(p->kh * p->kw) * g.chunks, g.kw = (int32_t)p->kw;
+        g.packed_rows = (int32_t)padded_rows(p->m);
+        g.sh = (int32_t)p->stride_h, g.sw = (int32_t)p->stride_w, g.dh = (int32_t)p->dil_h, g.dw = (int32_t)p->dil_w;
+        g.pad_top = (int32_t)p->pad_top, g.pad_left = (int32_t)p->pad_left;
+        g.act = p->act & (B200ML_EPI_RELU | B200ML_EPI_GELU | B200ML_EPI_SWISH);
+        g.y_nhwc = y_nhwc ? 1 : 0;
+        g.status = ctx->status_dev;
+        // the pixel box that covers the output with the fewest tiles; an element stride limits its extent (256 source elements)
+        int64_t best = INT64_MAX;
+        const int64_t max_w = ow < 128 ? ow : 128;
+        for (int64_t wb = max_w; wb >= 1; --wb) {
+            if ((wb - 1) * p->stride_w + 1 > 256) continue;
+            int64_t hb = oh < 128 / wb ? oh : 128 / wb;
+            while ((hb - 1) * p->stride_h + 1 > 256) --hb;
+            int64_t nb = wb == ow && hb == oh ? 128 / (wb * hb) : 1;
+            if (nb > n) nb = n;
+            const int64_t tiles = ceil_div(ow, wb) * ceil_div(oh, hb) * ceil_div(n, nb);
+            if (tiles < best) best = tiles, g.wb = (int32_t)wb, g.hb = (int32_t)hb, g.nb = (int32_t)nb;
+        }
+        g.tiles_w = (int32_t)ceil_div(ow, g.wb), g.tiles_h = (int32_t)ceil_div(oh, g.hb), g.tiles_n = (int32_t)ceil_div(n, g.nb);
+        const cuuint64_t es = sizeof(T);
+        const cuuint64_t dims[4] = {(cuuint64_t)cp, (cuuint64_t)p->w, (cuuint64_t)p->h, (cuuint64_t)n};
+        const cuuint64_t strides[3] = {(cuuint64_t)cp * es, (cuuint64_t)(cp * p->w) * es, (cuuint64_t)image * es};
+        const cuuint32_t box[4] = {(cuuint32_t)kc, (cuuint32_t)((g.wb - 1) * p->stride_w + 1), (cuuint32_t)((g.hb - 1) * p->stride_h + 1), (cuuint32_t)g.nb};
+        const cuuint32_t step[4] = {1, (cuuint32_t)p->stride_w, (cuuint32_t)p->stride_h, 1};
+        const CUtensorMapSwizzle swizzle = g.kcb == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (g.kcb == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+        CUtensorMap maps[2];
+        for (int part = 0; part < 2; ++part) {
+            if (part == PARTS) {
+                maps[1] = maps[0];
+                break;
+            }
+            const CUresult r = encode_tiled_cached(ctx, &maps[part], sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                                                   x + part * n * image, dims, strides, box, swizzle, step);
+            if (r != CUDA_SUCCESS) return fail(B200ML_ERR_CUDA, "cuTensorMapEncodeTiled(X channels-last) failed with CUresult %d", (int)r);
+        }
+        // Narrower channel blocks where the wide ones would leave half of the CTA slots idle; fp32 stages of 128 channels would
+        // leave room for one only.
+        const int64_t pixel_tiles = (int64_t)g.tiles_w * g.tiles_h * g.tiles_n;
+        int rc;
+        if (p->m <= 32) rc = launch_conv<T, 32>(ctx, maps[0], maps[1], g, s);
+        else if (p->m <= 64 || sizeof(T) == 4 || pixel_tiles * ceil_div(p->m, 128) < ctx->sm_count) rc = launch_conv<T, 64>(ctx, maps[0], maps[1], g, s);
+        else rc = launch_conv<__half, 128>(ctx, maps[0], maps[1], reinterpret_cast<ConvHArgs<__half>&>(g), s);
+        if (rc) return rc;
+    }
+    return B200ML_OK;
+}
+
+}  // namespace
+
+// Group 1, strides the TMA unit can make, reductions of 64 terms or more for fp32 (shorter ones are faster on the FMA pipe),
+// and enough work for the launches to pay (a 128 x 32 tile's worth of products).  The caller asks for the fp32 kernels that
+// read NCHW first.
+bool conv_nhwc_applies(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow) {
+    if (p->group != 1 || !ctx->encode_tiled) return false;
+    if (p->stride_h > 8 || p->stride_w > 8 || p->pad_top > 1024 || p->pad_left > 1024) return false;
+    if (p->n * p->m * oh * ow * p->c * p->kh * p->kw < (1ll << 19)) return false;
+    if (p->h * p->w >= (1ll << 31) || p->n * p->h * p->w * ceil_div(p->c, 8) >= (1ll << 35)) return false;
+    if (p->dtype == B200ML_F32) {
+        if ((p->act & (B200ML_CONV_X_NHWC | B200ML_CONV_Y_NHWC)) || p->c * p->kh * p->kw < 64) return false;
+        return padded_channels<float>(p->c) * p->h * p->w * 8 <= ctx->workspace_bytes / 2 && pack_elements<float>(p) * 4 <= ctx->workspace_bytes / 2;
+    }
+    if ((p->act & (B200ML_CONV_X_NHWC | B200ML_CONV_Y_NHWC)) && (!aligned16(p->x) || !aligned16(p->y))) return false;
+    // one image beside run-time weights
+    return padded_channels<__half>(p->c) * p->h * p->w * 2 <= ctx->workspace_bytes / 2 && pack_elements<__half>(p) * 2 <= ctx->workspace_bytes / 2;
+}
+
+int64_t conv_nhwc_pack_bytes(const b200ml_conv_params* p) {
+    return p->dtype == B200ML_F32 ? pack_elements<float>(p) * 4 : pack_elements<__half>(p) * 2;
+}
+
+int conv_nhwc_pack(const b200ml_ctx* ctx, const b200ml_conv_params* p, void* packed, cudaStream_t s) {
+    if (p->dtype == B200ML_F32) {
+        PrepareArgs<float> a{};
+        return launch_prepare<float>(ctx, a, p, static_cast<float*>(packed), s);
+    }
+    PrepareArgs<__half> a{};
+    return launch_prepare<__half>(ctx, a, p, static_cast<__half*>(packed), s);
+}
+
+int conv_nhwc(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow, cudaStream_t s) {
+    return p->dtype == B200ML_F32 ? conv_impl<float>(ctx, p, oh, ow, s) : conv_impl<__half>(ctx, p, oh, ow, s);
+}
+
+}  // namespace b200ml

@@ -1,4 +1,5 @@
-"""The fp16 implicit-GEMM convolution: channel chunks of 16 / 32 / 64 and ragged ones, channel blocks of each width, pixel boxes
+"""The implicit-GEMM convolution over channels-last operands, fp16 and fp32 (3 x TF32): channel chunks of 32 / 64 / 128 bytes and
+ragged ones, channel blocks of each width, pixel boxes
 over ragged and tiny images, strides, dilation, padding, a split reduction, gate / residual / activation, both layouts."""
 
 import pytest
@@ -18,7 +19,7 @@ CASES = [(4, 3, 40, 40, 16, 3, 2, 0, 1), (1, 16, 33, 17, 24, 3, 1, 1, 1), (3, 24
          (4, 8, 150, 131, 8, 7, 2, 3, 1), (9, 72, 5, 3, 40, 3, 1, 1, 1), (3, 32, 30, 30, 16, 2, 3, 0, 1), (1, 128, 64, 64, 96, 1, 2, 0, 1)]
 
 
-def _check(y, x, w, b, r, act, stride, pad, dil):
+def _check(y, x, w, b, r, act, stride, pad, dil, dtype=torch.float16):
     ref = F.conv2d(x.double(), w.double(), b.double(), stride, pad, dil)
     mag = F.conv2d(x.double().abs(), w.double().abs(), b.double().abs(), stride, pad, dil)
     if act == L.EPI_RELU:
@@ -26,57 +27,61 @@ def _check(y, x, w, b, r, act, stride, pad, dil):
     elif act == L.EPI_SWISH:
         ref = ref * torch.sigmoid(ref)
     ref = ref + r.double()
-    # fp32 accumulation (truncated adds: a few 2^-24 of the terms' magnitude per hundred of them), one fp16 rounding of the result
-    err, bound = (y.double() - ref).abs(), 4e-6 * mag + 2.0**-10 * ref.abs() + 1e-6
+    # fp32 accumulation (truncated adds: a few 2^-24 of the terms' magnitude per hundred of them; fp32 operands in 22 bits),
+    # one fp16 rounding of the result
+    err, bound = (y.double() - ref).abs(), 4e-6 * mag + (2.0**-10 * ref.abs() if dtype == torch.float16 else 0.0) + 1e-6
     assert bool((err <= bound).all()), "worst error / bound %.3g" % float((err / bound).max())
 
 
-def _inputs(case, seed):
+def _inputs(case, seed, dtype=torch.float16):
     n, c, h, w, m, k, stride, pad, dil = case
     gen = torch.Generator("cuda").manual_seed(seed)
 
     def rand(*s, scale=1.0):
-        return (torch.randn(*s, device="cuda", generator=gen) * scale).half()
+        return (torch.randn(*s, device="cuda", generator=gen) * scale).to(dtype)
 
     oh, ow = ((s + 2 * pad - dil * (k - 1) - 1) // stride + 1 for s in (h, w))
     return rand(n, c, h, w), rand(m, c, k, k, scale=(c * k * k)**-0.5), rand(m), rand(n, m, oh, ow)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("case", CASES)
-def test_conv_f16(case):
+def test_conv(case, dtype):
     n, c, h, w, m, k, stride, pad, dil = case
-    x, wt, b, r = _inputs(case, 3)
+    x, wt, b, r = _inputs(case, 3, dtype)
     for act, packed in ((0, False), (L.EPI_RELU, True), (L.EPI_SWISH, False)):
         args = dict(strides=(stride, stride), pads=(pad, ) * 4, dilations=(dil, dil))
         pw = K.conv_prepack(x.shape, wt, bias=b, **args) if packed else None
-        assert not packed or pw is not None
-        guard = torch.full((r.numel() + 64, ), 7.0, dtype=torch.float16, device="cuda")
+        assert not packed or pw is not None or (dtype == torch.float32 and c * k * k < 64)  # short fp32 reductions: another kernel
+        guard = torch.full((r.numel() + 64, ), 7.0, dtype=dtype, device="cuda")
         y = guard[:r.numel()].view(r.shape)
         K.conv2d(x, wt, y, bias=b, residual=r, act=act, packed_weight=pw, **args)
-        _check(y, x, wt, b, r, act, stride, pad, dil)
+        _check(y, x, wt, b, r, act, stride, pad, dil, dtype)
         assert bool((guard[r.numel():] == 7.0).all())
     assert L.get_context(0).device_status() == 0
 
 
-def test_conv_f16_gate():
-    case = (3, 40, 15, 15, 24, 1, 1, 0, 1)
-    x, wt, b, r = _inputs(case, 4)
-    gate = torch.rand(3, 40, 1, 1, device="cuda").half()
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_gate(dtype):
+    case = (3, 72, 15, 15, 24, 1, 1, 0, 1)
+    x, wt, b, r = _inputs(case, 4, dtype)
+    gate = torch.rand(3, 72, 1, 1, device="cuda").to(dtype)
     y = torch.empty_like(r)
     K.conv2d(x, wt, y, bias=b, gate=gate, residual=r)
-    _check(y, (x.float() * gate.float()).half(), wt, b, r, 0, 1, 0, 1)
+    _check(y, (x.float() * gate.float()).to(dtype), wt, b, r, 0, 1, 0, 1, dtype)
 
 
-def test_conv_f16_images_in_pieces():
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_images_in_pieces(dtype):
     """The channels-last copy of these images does not fit the scratch of the context: several launches."""
-    case = (11, 24, 40, 40, 16, 3, 1, 1, 1)
-    x, wt, b, r = _inputs(case, 5)
+    case = (11, 24, 9, 40, 16, 3, 1, 1, 1)
+    x, wt, b, r = _inputs(case, 5, dtype)
     y = torch.empty_like(r)
-    ctx = L.Context(0, workspace_bytes=4 * 24 * 40 * 40 * 2)
+    ctx = L.Context(0, workspace_bytes=200 << 10)
     with L.use_context(ctx):
         K.conv2d(x, wt, y, bias=b, residual=r, pads=(1, 1, 1, 1))
     torch.cuda.synchronize()
-    _check(y, x, wt, b, r, 0, 1, 1, 1)
+    _check(y, x, wt, b, r, 0, 1, 1, 1, dtype)
     assert ctx.device_status() == 0
 
 
