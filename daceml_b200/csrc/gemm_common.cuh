@@ -36,6 +36,19 @@ struct GemmArgs {
     long long* trace;  // per-CTA cycle counters, only written when built with B200ML_TRACE
 };
 
+}  // namespace gemm
+
+// Tile width and K split of the kernel for few output tiles (gemm_split.cu); bn == 0: not for it.
+struct SplitPlan {
+    int bn, split;
+};
+SplitPlan gemm_f16_split_plan(const b200ml_ctx* ctx, const b200ml_gemm_params* p, bool vec_ok);
+// `f32_rows`: args.c is float* and receives the finished rows in fp32 (a LayerNorm launch follows).
+int gemm_f16_split(const b200ml_ctx* ctx, const b200ml_gemm_params* p, gemm::GemmArgs& args, const SplitPlan& plan, bool f32_rows, cudaStream_t stream);
+int layernorm_f32_rows(const float* x, const __half* gamma, const __half* beta, __half* y, int m, int n, int64_t ldy, float eps, cudaStream_t stream);
+
+namespace gemm {
+
 #ifdef B200ML_TRACE
 #define TRACE_T0() const long long _t0 = clock64()
 #define TRACE_ADD(var) var += clock64() - _t0

@@ -1,0 +1,413 @@
+// fp16 GEMM for products with few output tiles: C[M, N] = epilogue(alpha * A[M, K] . B), fp32 accumulate on tcgen05.
+//
+// The persistent kernels (gemm_tc.cu, gemm_tc2.cu) give every 128 x 256 (or 256 x 256) tile to one CTA (pair), which takes in
+// operands at some 100 bytes per cycle: with 3 to 40 such tiles most SMs idle and the few busy ones stream K from end to end
+// (77 x 768 x 3072: three CTAs, 20 us).  Here a tile is 128 x BN (64 or 128) and K is split over a cluster of up to eight
+// CTAs: the partial tiles are parked in shared memory, every CTA adds up its share of the rows through distributed shared
+// memory (in rank order: the same sum on every run) and finishes them.
+// A CTA holds less than half of an SM's shared memory, so the CTAs of the next kernel in a chain become resident while this
+// one runs and fetch their constant weights (b_early) under it: a chain of small products is then bound by the dependency
+// hand-overs, not by the weights.
+#include "gemm_common.cuh"
+
+namespace b200ml {
+
+using namespace gemm;
+
+namespace {
+
+constexpr int SP_THREADS = 64 + 256;  // TMA warp, MMA warp, eight epilogue warps
+
+template <int BN>
+struct SplitSmem {
+    static constexpr int B_TILE_BYTES = BN * BK * 2;
+    static constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
+    static constexpr int STAGES = BN == 64 ? 4 : 3;  // 96 KB
+    static constexpr int PART_LD = BN + 4;           // floats between rows of the parked tile: 16-byte rows, no bank conflicts
+    static constexpr int TOTAL = STAGES * STAGE_BYTES + 256 + 1024;
+    static_assert(BM * PART_LD * 4 <= STAGES * STAGE_BYTES, "the parked tile lies over the pipeline stages");
+};
+
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t local_addr, uint32_t rank) {
+    uint32_t raddr;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(raddr) : "r"(local_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(raddr) : "memory");
+    return v;
+}
+
+// Eight columns of one row: alpha, bias, activation, residual, one 16-byte store (two of fp32).
+template <bool F32>
+__device__ __forceinline__ void split_finish8(const GemmArgs& g, float (&v)[8], bool bias, const uint4& bq, bool res, const uint4& rq, int64_t at) {
+    if (g.alpha != 1.0f) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] *= g.alpha;
+    }
+    if (bias) {
+        float b[8];
+        unpack8(bq, b);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = fmaf(g.bias_scale, b[j], v[j]);
+    }
+    if (!F32 && (g.epilogue & B200ML_EPI_GELU) && !res) {
+        *reinterpret_cast<uint4*>(g.c + at) = gelu_pack8(v);
+        return;
+    }
+    if (g.epilogue & (B200ML_EPI_RELU | B200ML_EPI_GELU | B200ML_EPI_SWISH)) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = apply_act_f16(v[j], g.epilogue);
+    }
+    if (res) {
+        float q[8];
+        unpack8(rq, q);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = fmaf(g.residual_scale, q[j], v[j]);
+    }
+    if (F32) {
+        float4* out = reinterpret_cast<float4*>(reinterpret_cast<float*>(g.c) + at);
+        out[0] = make_float4(v[0], v[1], v[2], v[3]);
+        out[1] = make_float4(v[4], v[5], v[6], v[7]);
+    } else {
+        *reinterpret_cast<uint4*>(g.c + at) = pack8(v);
+    }
+}
+
+// The eight columns at `at` of the parked tiles of all ranks, summed in rank order (the same sum on every run); the loads of
+// all ranks are in flight together.
+template <int SPLIT>
+__device__ __forceinline__ void sum_ranks(uint32_t at, float (&v)[8]) {
+    float4 x[SPLIT], y[SPLIT];
+#pragma unroll
+    for (int q = 0; q < SPLIT; ++q) x[q] = ld_cluster_v4(at, q), y[q] = ld_cluster_v4(at + 16, q);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+#pragma unroll
+    for (int q = 0; q < SPLIT; ++q)
+        v[0] += x[q].x, v[1] += x[q].y, v[2] += x[q].z, v[3] += x[q].w, v[4] += y[q].x, v[5] += y[q].y, v[6] += y[q].z, v[7] += y[q].w;
+}
+
+template <int BN, bool B_MN, bool F32>
+__global__ void __launch_bounds__(SP_THREADS, 2)
+gemm_f16_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmArgs args, const int split) {
+    using S = SplitSmem<BN>;
+    constexpr int STAGES = S::STAGES;
+    constexpr uint32_t IDESC = ptx::make_idesc_f16(BM, BN, 0, B_MN ? 1 : 0);
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * S::STAGE_BYTES);
+    uint64_t* empty_bar = full_bar + STAGES;
+    uint64_t* acc_bar = empty_bar + STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = split > 1 ? static_cast<int>(ptx::cluster_ctarank()) : 0;
+    const int tile = blockIdx.x / split;
+    const int m0 = (tile % args.tiles_m) * BM, n0 = (tile / args.tiles_m) * BN;
+    const int num_kb = (args.k + BK - 1) / BK;
+    const int kb_per = (num_kb + split - 1) / split;
+    const int kb_begin = rank * kb_per < num_kb ? rank * kb_per : num_kb;
+    const int nk = (kb_begin + kb_per < num_kb ? kb_begin + kb_per : num_kb) - kb_begin;  // may be 0
+
+    if (warp == 0 && lane == 0) {
+        ptx::prefetch_tensormap(&tmap_a);
+        ptx::prefetch_tensormap(&tmap_b);
+    }
+    if (warp == 1) {
+        if (lane == 0) {
+            for (int s = 0; s < STAGES; ++s) {
+                ptx::mbar_init(&full_bar[s], 1);
+                ptx::mbar_init(&empty_bar[s], 1);
+            }
+            ptx::mbar_init(acc_bar, 1);
+            ptx::fence_mbar_init();
+        }
+        __syncwarp();
+        ptx::tmem_alloc(tmem_slot, BN);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    pdl_launch_dependents();  // after the allocation: an early CTA of the next kernel cannot take this CTA's tensor memory
+    ptx::tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        // ------------------------------ TMA producer ------------------------------
+        if (ptx::elect_one()) {
+            auto load_b = [&](int i, int stage) {
+                uint8_t* sb = smem + stage * S::STAGE_BYTES + A_TILE_BYTES;
+                ptx::mbar_expect_tx(&full_bar[stage], S::STAGE_BYTES);
+                const int k = (kb_begin + i) * BK;
+                if (B_MN) {
+#pragma unroll
+                    for (int j = 0; j < BN / 64; ++j) ptx::tma_load_4d(sb + j * (64 * BK * 2), &tmap_b, &full_bar[stage], n0 + j * 64, k, 0, 0);
+                } else {
+                    ptx::tma_load_4d(sb, &tmap_b, &full_bar[stage], k, n0, 0, 0);
+                }
+            };
+            const int early = args.b_early ? (nk < STAGES ? nk : STAGES) : 0;
+            for (int i = 0; i < early; ++i) load_b(i, i);  // constant weights: before the dependency wait
+            pdl_wait();
+            int stage = 0;
+            uint32_t phase = 0;
+            for (int i = 0; i < nk; ++i) {
+                if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1)) {
+                    atomicExch(args.status, DEV_TIMEOUT_PRODUCER);
+                    break;
+                }
+                if (i >= early) load_b(i, stage);
+                ptx::tma_load_4d(smem + stage * S::STAGE_BYTES, &tmap_a, &full_bar[stage], (kb_begin + i) * BK, m0, 0, 0);
+                if (++stage == STAGES) stage = 0, phase ^= 1;
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // ------------------------------ MMA issuer ------------------------------
+        if (ptx::elect_one()) {
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int i = 0; i < nk; ++i) {
+                if (!ptx::mbar_wait(&full_bar[stage], phase)) {
+                    atomicExch(args.status, DEV_TIMEOUT_MMA);
+                    ok = false;
+                    break;
+                }
+                ptx::tc_fence_after();
+                const uint32_t a_addr = ptx::smem_u32(smem + stage * S::STAGE_BYTES), b_addr = a_addr + A_TILE_BYTES;
+#pragma unroll
+                for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+                    const uint64_t a_desc = ptx::make_smem_desc_sw128(a_addr + kk * (UMMA_K * 2), 16, 1024);
+                    const uint64_t b_desc = B_MN ? ptx::make_smem_desc_sw128(b_addr + kk * (UMMA_K * 128), 64 * BK * 2, 1024)
+                                                 : ptx::make_smem_desc_sw128(b_addr + kk * (UMMA_K * 2), 16, 1024);
+                    ptx::mma_f16_ss(tmem_base, a_desc, b_desc, IDESC, (i | kk) != 0 ? 1u : 0u);
+                }
+                ptx::mma_commit(&empty_bar[stage]);
+                if (++stage == STAGES) stage = 0, phase ^= 1;
+            }
+            if (ok && nk > 0) ptx::mma_commit(acc_bar);
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------ accumulator -> parked tile ------------------------------
+        pdl_wait();  // the residual may be a predecessor's
+        const bool has_bias = (args.epilogue & B200ML_EPI_BIAS) && args.bias, has_res = (args.epilogue & B200ML_EPI_RESIDUAL) && args.residual;
+        // where this thread's first finished values will lie: their bias and residual are fetched while the products run
+        constexpr int C8 = BN / 8, ROWS_PER_PASS = 256 / C8;
+        const int t = threadIdx.x - 64;
+        const int rows = args.m - m0 < BM ? args.m - m0 : BM;
+        const int share = (rows + split - 1) / split;
+        const int end = (rank + 1) * share < rows ? (rank + 1) * share : rows;
+        const int col = n0 + (t % C8) * 8;
+        int r = rank * share + t / C8;
+        const bool col_ok = col < args.n;
+        uint4 bq = make_uint4(0, 0, 0, 0), rq = make_uint4(0, 0, 0, 0);
+        if (has_bias && col_ok) bq = __ldg(reinterpret_cast<const uint4*>(args.bias + col));
+        if (has_res && col_ok && r < end) rq = __ldg(reinterpret_cast<const uint4*>(args.residual + static_cast<int64_t>(m0 + r) * args.ldr + col));
+
+        float* partial = reinterpret_cast<float*>(smem);
+        const int quarter = warp & 3, half = (warp - 2) >> 2, row = quarter * 32 + lane;
+        bool ok = true;
+        if (nk > 0 && !ptx::mbar_wait(acc_bar, 0)) {
+            if (lane == 0) atomicExch(args.status, DEV_TIMEOUT_EPILOGUE);
+            ok = false;
+        }
+        __syncwarp();
+        ptx::tc_fence_after();
+#pragma unroll 1
+        for (int c = half * (BN / 2); ok && c < (half + 1) * (BN / 2); c += 32) {
+            if (m0 + quarter * 32 >= args.m || n0 + c >= args.n) break;  // warp-uniform
+            uint32_t acc[32];
+            if (nk > 0) {
+                ptx::tmem_ld_32x32b_x32(tmem_base + c + (static_cast<uint32_t>(quarter * 32) << 16), acc);
+                ptx::tmem_ld_wait();
+            } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) acc[j] = 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                *reinterpret_cast<uint4*>(partial + row * S::PART_LD + c + 4 * j) = make_uint4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+        }
+        ptx::tc_fence_before();
+        // ------------------------------ this CTA's share of the rows ------------------------------
+        if (split > 1) ptx::cluster_sync_acq_rel();
+        else asm volatile("bar.sync 1, 256;" ::: "memory");
+        const uint32_t part_addr = ptx::smem_u32(smem);
+        if (col_ok) {
+            for (; r < end; r += ROWS_PER_PASS) {
+                const uint32_t at = part_addr + (r * S::PART_LD + (t % C8) * 8) * 4;
+                float v[8];
+                switch (split) {
+                    case 1: {
+                        const float4 x = *reinterpret_cast<const float4*>(partial + r * S::PART_LD + (t % C8) * 8);
+                        const float4 y = *reinterpret_cast<const float4*>(partial + r * S::PART_LD + (t % C8) * 8 + 4);
+                        v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+                        break;
+                    }
+                    case 2: sum_ranks<2>(at, v); break;
+                    case 4: sum_ranks<4>(at, v); break;
+                    default: sum_ranks<8>(at, v); break;
+                }
+                split_finish8<F32>(args, v, has_bias, bq, has_res, rq, static_cast<int64_t>(m0 + r) * args.ldc + col);
+                if (has_res && r + ROWS_PER_PASS < end)
+                    rq = __ldg(reinterpret_cast<const uint4*>(args.residual + static_cast<int64_t>(m0 + r + ROWS_PER_PASS) * args.ldr + col));
+            }
+        }
+    }
+    if (warp < 2 && split > 1) ptx::cluster_sync_acq_rel();  // the producer and MMA warps' part of the barrier above
+    if (split > 1) ptx::cluster_sync_acq_rel();  // no CTA leaves while a peer may still read its partial tile
+    ptx::tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        ptx::tc_fence_after();
+        if (*reinterpret_cast<volatile int32_t*>(args.status) != DEV_OK) {
+            for (int i = 0; i < 200; ++i) __nanosleep(1000);  // a wait gave up: let copies and MMAs in flight land
+        }
+        ptx::tmem_dealloc(tmem_base, BN);
+    }
+}
+
+template <int BN, bool B_MN, bool F32>
+int launch_split(const b200ml_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs& args, int split, cudaStream_t stream) {
+    using S = SplitSmem<BN>;
+    auto kernel = gemm_f16_split_kernel<BN, B_MN, F32>;
+    static bool configured[64] = {};  // per instantiation and device
+    if (!configured[ctx->device & 63]) {
+        B200ML_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
+        configured[ctx->device & 63] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(args.num_tiles * split));
+    cfg.blockDim = dim3(SP_THREADS);
+    cfg.dynamicSmemBytes = S::TOTAL;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = split, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    B200ML_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, args, split));
+    return check_launch("gemm_f16_split");
+}
+
+// LayerNorm of fp32 rows into fp16: a warp per row, the row in registers (a lane holds up to four pieces of eight columns),
+// mean first, then the squared deviations.  Bound by latency: it runs over at most a few thousand rows that were just written.
+template <int PIECES>
+__global__ void __launch_bounds__(128) layernorm_f32_rows_kernel(const float* __restrict__ x, const __half* __restrict__ gamma, const __half* __restrict__ beta,
+                                                                 __half* __restrict__ y, int m, int n, int64_t ldy, float eps) {
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, row = blockIdx.x * 4 + (threadIdx.x >> 5);
+    uint4 gq[PIECES], bq[PIECES];
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {  // constants: before the dependency wait
+        const int c = (lane + 32 * i) * 8;
+        gq[i] = gamma && c < n ? __ldg(reinterpret_cast<const uint4*>(gamma + c)) : make_uint4(0, 0, 0, 0);
+        bq[i] = beta && c < n ? __ldg(reinterpret_cast<const uint4*>(beta + c)) : make_uint4(0, 0, 0, 0);
+    }
+    pdl_wait();
+    if (row >= m) return;
+    float v[PIECES][8];
+    float s = 0.0f;
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+        const int c = (lane + 32 * i) * 8;
+        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+        if (c < n) {
+            const float4* p = reinterpret_cast<const float4*>(x + static_cast<int64_t>(row) * n + c);
+            a = p[0], b = p[1];
+        }
+        v[i][0] = a.x, v[i][1] = a.y, v[i][2] = a.z, v[i][3] = a.w, v[i][4] = b.x, v[i][5] = b.y, v[i][6] = b.z, v[i][7] = b.w;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s += v[i][j];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const float mean = s / n;
+    float q = 0.0f;
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i)
+        if ((lane + 32 * i) * 8 < n) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) q = fmaf(v[i][j] - mean, v[i][j] - mean, q);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    const float rstd = rsqrtf(q / n + eps);
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+        const int c = (lane + 32 * i) * 8;
+        if (c >= n) break;
+        float gf[8], bf[8], o[8];
+        unpack8(gq[i], gf), unpack8(bq[i], bf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float t = (v[i][j] - mean) * rstd;
+            o[j] = gamma ? fmaf(t, gf[j], bf[j]) : t + bf[j];
+        }
+        *reinterpret_cast<uint4*>(y + static_cast<int64_t>(row) * ldy + c) = pack8(o);
+    }
+}
+
+template <bool F32>
+int launch_plan(const b200ml_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, bool b_mn, GemmArgs& args, const SplitPlan& plan, cudaStream_t stream) {
+    if (b_mn)
+        return plan.bn == 64 ? launch_split<64, true, F32>(ctx, ta, tb, args, plan.split, stream) : launch_split<128, true, F32>(ctx, ta, tb, args, plan.split, stream);
+    return plan.bn == 64 ? launch_split<64, false, F32>(ctx, ta, tb, args, plan.split, stream) : launch_split<128, false, F32>(ctx, ta, tb, args, plan.split, stream);
+}
+
+}  // namespace
+
+// How the split kernel would cut this product; bn == 0: the persistent kernels take it.  The lines come from timing both on
+// N, K of 256 to 4096 and 8 to 6534 rows:
+//   * two CTAs fit on an SM, so up to 2 x 148 tiles of 128 x 64 are one wave (2048 x 768 x 768: 12.5 us persistent, 7.3 split;
+//     1024 x 3072 x 768, 384 tiles: 10.9 and 12.9);
+//   * past that, 128-wide tiles of one wave win while K is short (4096 x 768 x 768: 12.9 and 10.5; K = 3072: 24.7 and 24.7);
+//   * K is split when that saves more k-blocks (0.155 us each) than the reduction costs (about 1.2 us, more with more rows
+//     per CTA and with eight ranks), on at most 96 CTAs (77 x 768 x 3072: 11.0 us unsplit, 6.3 with four).
+SplitPlan gemm_f16_split_plan(const b200ml_ctx* ctx, const b200ml_gemm_params* p, bool vec_ok) {
+    SplitPlan s{0, 1};
+    if (!vec_ok || p->n % 8 != 0 || p->batch_outer * p->batch_inner != 1) return s;
+    const int64_t tm = ceil_div(p->m, BM), t64 = tm * ceil_div(p->n, 64), t128 = tm * ceil_div(p->n, 128);
+    const int64_t slots = 2 * (int64_t)ctx->sm_count;
+    if (t64 > slots) {
+        if (t128 <= slots && p->k <= 1024) s.bn = 128;
+        return s;
+    }
+    s.bn = 64;
+    const int64_t rows = p->m < BM ? p->m : BM;
+    const float cost[3] = {1.2f, rows > 96 ? 2.4f : 1.2f, rows > 96 ? 4.5f : (rows > 32 ? 2.6f : 1.4f)};
+    const float kb = 0.155f * ceil_div(p->k, BK);
+    float best = kb;
+    for (int i = 0; i < 3; ++i) {
+        const int split = 2 << i;
+        if (t64 * split * 3 > (int64_t)ctx->sm_count * 2 || ceil_div(p->k, BK) < split) break;
+        if (kb / split + cost[i] < best) best = kb / split + cost[i], s.split = split;
+    }
+    return s;
+}
+
+int gemm_f16_split(const b200ml_ctx* ctx, const b200ml_gemm_params* p, GemmArgs& args, const SplitPlan& plan, bool f32_rows, cudaStream_t stream) {
+    args.tiles_m = (int32_t)ceil_div(p->m, BM);
+    args.tiles_n = (int32_t)ceil_div(p->n, plan.bn);
+    args.num_tiles = args.tiles_m * args.tiles_n;
+    CUtensorMap ta, tb;
+    int rc = make_tmap(ctx, &ta, p->a, p->k, p->m, p->lda, 1, 0, 1, 0, BK, BM, "A");
+    if (rc) return rc;
+    const bool b_mn = p->b_layout == 0;
+    rc = b_mn ? make_tmap(ctx, &tb, p->b, p->n, p->k, p->ldb, 1, 0, 1, 0, 64, BK, "B") : make_tmap(ctx, &tb, p->b, p->k, p->n, p->ldb, 1, 0, 1, 0, BK, plan.bn, "B");
+    if (rc) return rc;
+    return f32_rows ? launch_plan<true>(ctx, ta, tb, b_mn, args, plan, stream) : launch_plan<false>(ctx, ta, tb, b_mn, args, plan, stream);
+}
+
+int layernorm_f32_rows(const float* x, const __half* gamma, const __half* beta, __half* y, int m, int n, int64_t ldy, float eps, cudaStream_t stream) {
+    const dim3 grid((unsigned)ceil_div(m, 4)), block(128);
+    if (n <= 256) B200ML_CUDA(launch_pdl(layernorm_f32_rows_kernel<1>, grid, block, 0, stream, x, gamma, beta, y, m, n, ldy, eps));
+    else if (n <= 512) B200ML_CUDA(launch_pdl(layernorm_f32_rows_kernel<2>, grid, block, 0, stream, x, gamma, beta, y, m, n, ldy, eps));
+    else B200ML_CUDA(launch_pdl(layernorm_f32_rows_kernel<4>, grid, block, 0, stream, x, gamma, beta, y, m, n, ldy, eps));
+    return check_launch("layernorm_f32_rows");
+}
+
+}  // namespace b200ml

@@ -104,9 +104,9 @@ class DaceModule(nn.Module):
 
             self.prepend_post_onnx_hook("make_transients_outputs", transients_outputs)
 
-        if self.auto_optimize:
+        if self.auto_optimize:  # the hook must not hold the module: a module that is dropped gives its memory back at once
             self.append_post_onnx_hook(
-                "auto_optimize", lambda dace_module: utils.auto_optimize(dace_module.dace_model.sdfg, True, simplify=self.simplify))
+                "auto_optimize", lambda dace_module: utils.auto_optimize(dace_module.dace_model.sdfg, True, simplify=simplify))
 
         if dummy_inputs is not None:
             self.function = self._initialize_sdfg(dummy_inputs)

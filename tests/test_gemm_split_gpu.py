@@ -1,0 +1,61 @@
+"""The fp16 GEMM for few output tiles: both tile widths, every split of K (also with empty shares), ragged rows, columns and K,
+both layouts of B, the epilogue forms; and LayerNorm behind it, against the fused kernel's definition."""
+import pytest
+import torch
+
+from daceml_b200 import kernels as K
+from daceml_b200 import lib as L
+
+pytestmark = pytest.mark.gpu
+
+# m, n, k: the 128-row edge; one, two, four and eight shares of K (tiles of 64 columns); 128-column tiles; ragged N and K
+SIZES = [(9, 64, 64), (77, 768, 768), (128, 768, 3072), (129, 2304, 768), (16, 1024, 4096), (20, 72, 1000), (300, 200, 136), (403, 1024, 2048),
+         (2048, 768, 768), (4096, 768, 768), (3000, 1024, 264)]
+
+
+def _bound(ref, mag):
+    # fp32 accumulation of fp16 products (truncated adds), one rounding of the result, one of the activation's half2 form
+    return 4e-6 * mag + 2.0**-9 * ref.abs() + 2e-3
+
+
+@pytest.mark.parametrize("b_layout", [0, 1])
+@pytest.mark.parametrize("m, n, k", SIZES)
+def test_split_gemm(m, n, k, b_layout):
+    gen = torch.Generator("cuda").manual_seed(5)
+
+    def rand(*s, scale=1.0):
+        return (torch.randn(*s, device="cuda", generator=gen) * scale).half()
+
+    a, b, bias, res = rand(m, k), rand(k, n, scale=k**-0.5), rand(n), rand(m, n)
+    bl = b.t().contiguous() if b_layout else b
+    pre = a.double() @ b.double() + bias.double()
+    mag = a.double().abs() @ b.double().abs()
+    for act, residual in ((0, None), (L.EPI_GELU, None), (L.EPI_RELU, res), (L.EPI_GELU, res)):
+        guard = torch.full((m + 2, n), 7.0, dtype=torch.float16, device="cuda")
+        K.gemm(a, bl, guard[:m], b_layout=b_layout, bias=bias, residual=residual, act=act, b_constant=residual is not None)
+        ref = {0: pre, L.EPI_RELU: pre.relu(), L.EPI_GELU: torch.nn.functional.gelu(pre)}[act]
+        ref = ref + (residual.double() if residual is not None else 0.0)
+        err, bound = (guard[:m].double() - ref).abs(), _bound(ref, mag)
+        assert bool((err <= bound).all()), "act %d: worst error / bound %.3g" % (act, float((err / bound).max()))
+        assert bool((guard[m:] == 7.0).all())
+    assert L.get_context(0).device_status() == 0
+
+
+@pytest.mark.parametrize("m, n, k", [(5, 256, 64), (77, 512, 1024), (130, 768, 768), (1024, 1024, 512), (4096, 768, 128), (3000, 768, 200)])
+def test_layernorm_behind_a_gemm(m, n, k):
+    gen = torch.Generator("cuda").manual_seed(6)
+
+    def rand(*s, scale=1.0):
+        return (torch.randn(*s, device="cuda", generator=gen) * scale).half()
+
+    a, b, bias, res, gamma, beta = rand(m, k), rand(n, k, scale=k**-0.5), rand(n), rand(m, n), rand(n), rand(n)
+    pre = a.double() @ b.double().t() + bias.double() + res.double()
+    ref = torch.nn.functional.layer_norm(pre, (n, ), gamma.double(), beta.double(), 1e-12)
+    guard = torch.full((m + 2, n), 7.0, dtype=torch.float16, device="cuda")
+    K.gemm(a, b, guard[:m], b_layout=1, bias=bias, residual=res, ln=(gamma, beta, 1e-12))
+    err = (guard[:m].double() - ref).abs()
+    # statistics and values in fp32 (1e-5 of a row's unit deviation times gamma), one rounding of the result
+    bound = 2.0**-10 * ref.abs() + 2e-5 * (1.0 + gamma.double().abs()) + 1e-5
+    assert bool((err <= bound).all()), "worst error / bound %.3g" % float((err / bound).max())
+    assert bool((guard[m:] == 7.0).all())
+    assert L.get_context(0).device_status() == 0
