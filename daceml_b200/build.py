@@ -11,6 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libdaceml_b200.so")
+DISPATCH_PATH = os.path.join(LIB_DIR, "_dispatch.so")
 
 SOURCES = ["api.cu", "gemm_tc.cu", "gemm_tc2.cu", "gemm_ln.cu", "gemm_split.cu", "gemm_f32.cu", "rowwise.cu", "elementwise.cu", "indexing.cu", "conv.cu", "conv1x1_tc.cu", "conv_igemm.cu", "conv_nhwc.cu", "attention.cu", "diagnostics.cu", "peer.cu", "plan.cu"]
 
@@ -42,8 +43,32 @@ def needs_build():
     return any(os.path.getmtime(f) > built for f in _deps())
 
 
+def build_dispatch(force=False, verbose=False):
+    """Compiles ``csrc/dispatch.cpp``, the native call of compiled modules, against the installed torch (host code only)."""
+    import sysconfig
+    import torch
+    src = os.path.join(CSRC, "dispatch.cpp")
+    if not force and os.path.exists(DISPATCH_PATH) and os.path.getmtime(DISPATCH_PATH) >= os.path.getmtime(src):
+        return DISPATCH_PATH
+    os.makedirs(LIB_DIR, exist_ok=True)
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(find_nvcc()))
+    includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    libs = os.path.join(root, "lib")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-w", *["-I" + i for i in includes],
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), src, "-o", DISPATCH_PATH, "-L" + libs, "-Wl,-rpath," + libs,
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    subprocess.run(cmd, check=True)
+    return DISPATCH_PATH
+
+
 def build(force=False, verbose=False, ptxas_info=False):
-    """Compiles every ``.cu`` under ``csrc/`` into one shared library.  Returns its path."""
+    """Compiles every ``.cu`` under ``csrc/`` into one shared library, and the native call module beside it.  Returns the
+    library's path."""
+    build_dispatch(force, verbose)
     if not force and not needs_build():
         return LIB_PATH
     nvcc = find_nvcc()

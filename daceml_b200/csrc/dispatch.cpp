@@ -1,0 +1,208 @@
+// The call of a compiled module from Python, natively: checks the arguments, allocates the outputs and runs the launch plan
+// (plan.cu).  The counterpart of the reference's generated torch extension (daceml/torch/dispatchers/cpp_torch_extension.py),
+// built once for all modules.
+//
+// In Python the same steps cost 8-10 us per call (shape and type comparisons, torch.empty, building the address array, the
+// foreign-function call), more than a small module's launches; here about 1.5 us, most of it the output allocation.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+
+#include <vector>
+
+namespace {
+
+using PlanRun = int (*)(const void* plan, void* ctx, void* const* slots, int32_t n_slots, void* stream);
+
+struct Spec {
+    at::ScalarType dtype;
+    std::vector<int64_t> shape;
+};
+
+struct Call {
+    PlanRun run;
+    void* plan;
+    void* ctx;
+    c10::DeviceIndex device;
+    std::vector<Spec> inputs, outputs;
+    std::vector<int32_t> order;  // slot -> input (or number of inputs + output)
+    c10::DispatchKeySet plain;   // dispatch keys of an ordinary tensor on the device
+};
+
+struct PlannedCall {
+    PyObject_HEAD
+    vectorcallfunc vectorcall;
+    Call* call;
+    PyObject* keep;      // the plan and context objects
+    PyObject* on_error;  // called with the status code
+};
+
+// One call; a new reference to the result, Py_NotImplemented where the arguments need the general path.
+PyObject* planned_vectorcall(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
+    const PlannedCall* pc = reinterpret_cast<PlannedCall*>(self);
+    const Call& c = *pc->call;
+    const size_t n = PyVectorcall_NARGS(nargsf), n_out = c.outputs.size();
+    constexpr size_t MAX_SLOTS = 64;
+    if (kwnames || n != c.inputs.size() || n + n_out > MAX_SLOTS) Py_RETURN_NOTIMPLEMENTED;
+    // whoever looks at operators (modes, tracing) gets the registered operator instead
+    if (c10::impl::TorchDispatchModeTLS::stack_len() != 0 || at::impl::torch_function_mode_enabled() || torch::jit::tracer::isTracing())
+        Py_RETURN_NOTIMPLEMENTED;
+    void* addr[MAX_SLOTS];
+    for (size_t i = 0; i < n; ++i) {
+        if (!THPVariable_CheckExact(args[i])) Py_RETURN_NOTIMPLEMENTED;
+        const at::Tensor& t = THPVariable_Unpack(args[i]);
+        const Spec& s = c.inputs[i];
+        if ((t.key_set().raw_repr() & ~c.plain.raw_repr()) != 0 || !t.is_cuda() || t.get_device() != c.device || t.scalar_type() != s.dtype ||
+            !t.sizes().equals(s.shape) || !t.is_contiguous())
+            Py_RETURN_NOTIMPLEMENTED;
+        addr[i] = t.data_ptr();
+    }
+    try {
+        at::Tensor out[MAX_SLOTS];
+        const c10::Device device(c10::kCUDA, c.device);
+        for (size_t i = 0; i < n_out; ++i) {
+            out[i] = at::Tensor(at::detail::empty_cuda(c.outputs[i].shape, c.outputs[i].dtype, device, c10::nullopt));
+            addr[n + i] = out[i].data_ptr();
+        }
+        void* slots[MAX_SLOTS];
+        for (size_t i = 0; i < c.order.size(); ++i) slots[i] = addr[c.order[i]];
+        void* stream = c10::cuda::getCurrentCUDAStream(c.device).stream();
+        int rc;
+        Py_BEGIN_ALLOW_THREADS;
+        rc = c.run(c.plan, c.ctx, slots, static_cast<int32_t>(c.order.size()), stream);
+        Py_END_ALLOW_THREADS;
+        if (rc != 0) {
+            PyObject* r = PyObject_CallFunction(pc->on_error, "i", rc);
+            if (r) {
+                Py_DECREF(r);
+                PyErr_Format(PyExc_RuntimeError, "launch plan failed with status %d", rc);
+            }
+            return nullptr;
+        }
+        if (n_out == 1) return THPVariable_Wrap(std::move(out[0]));
+        PyObject* tuple = PyTuple_New(static_cast<Py_ssize_t>(n_out));
+        if (!tuple) return nullptr;
+        for (size_t i = 0; i < n_out; ++i) {
+            PyObject* w = THPVariable_Wrap(std::move(out[i]));
+            if (!w) {
+                Py_DECREF(tuple);
+                return nullptr;
+            }
+            PyTuple_SET_ITEM(tuple, static_cast<Py_ssize_t>(i), w);
+        }
+        return tuple;
+    } catch (const c10::OutOfMemoryError& e) {
+        PyObject* torch = PyImport_ImportModule("torch");
+        PyObject* type = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
+        PyErr_Clear();
+        PyErr_SetString(type ? type : PyExc_RuntimeError, e.what_without_backtrace());
+        Py_XDECREF(type);
+        Py_XDECREF(torch);
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+    }
+    return nullptr;
+}
+
+bool read_specs(PyObject* list, std::vector<Spec>* out) {
+    const Py_ssize_t n = PySequence_Size(list);
+    for (Py_ssize_t i = 0; i < n; ++i) {
+        PyObject* pair = PySequence_GetItem(list, i);
+        PyObject *shape = nullptr, *dtype = nullptr;
+        const bool ok = pair && PyArg_ParseTuple(pair, "OO", &shape, &dtype) && THPDtype_Check(dtype);
+        if (!ok) {
+            Py_XDECREF(pair);
+            if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "expected (shape, dtype) pairs");
+            return false;
+        }
+        Spec s;
+        s.dtype = reinterpret_cast<THPDtype*>(dtype)->scalar_type;
+        for (Py_ssize_t d = 0; d < PySequence_Size(shape); ++d) {
+            PyObject* e = PySequence_GetItem(shape, d);
+            s.shape.push_back(PyLong_AsLongLong(e));
+            Py_XDECREF(e);
+        }
+        out->push_back(std::move(s));
+        Py_DECREF(pair);
+    }
+    return !PyErr_Occurred();
+}
+
+// PlannedCall(run address, plan handle, context handle, device, [(shape, dtype)] inputs, outputs, [slot order], keep, on_error)
+PyObject* planned_new(PyTypeObject* type, PyObject* args, PyObject*) {
+    unsigned long long run, plan, ctx;
+    int device;
+    PyObject *inputs, *outputs, *order, *keep, *on_error;
+    if (!PyArg_ParseTuple(args, "KKKiOOOOO", &run, &plan, &ctx, &device, &inputs, &outputs, &order, &keep, &on_error)) return nullptr;
+    Call* c = new Call{reinterpret_cast<PlanRun>(run), reinterpret_cast<void*>(plan), reinterpret_cast<void*>(ctx), static_cast<c10::DeviceIndex>(device), {}, {}, {}, {}};
+    bool ok = read_specs(inputs, &c->inputs) && read_specs(outputs, &c->outputs);
+    for (Py_ssize_t i = 0; ok && i < PySequence_Size(order); ++i) {
+        PyObject* e = PySequence_GetItem(order, i);
+        const long long v = PyLong_AsLongLong(e);
+        Py_XDECREF(e);
+        ok = v >= 0 && v < static_cast<long long>(c->inputs.size() + c->outputs.size());
+        c->order.push_back(static_cast<int32_t>(v));
+    }
+    if (!ok) {
+        delete c;
+        if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "bad slot order");
+        return nullptr;
+    }
+    try {
+        c->plain = at::Tensor(at::detail::empty_cuda({0}, at::kFloat, c10::Device(c10::kCUDA, c->device), c10::nullopt)).key_set();
+    } catch (const std::exception& e) {
+        delete c;
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+    PlannedCall* self = reinterpret_cast<PlannedCall*>(type->tp_alloc(type, 0));
+    if (!self) {
+        delete c;
+        return nullptr;
+    }
+    self->vectorcall = planned_vectorcall;
+    self->call = c;
+    Py_INCREF(keep);
+    self->keep = keep;
+    Py_INCREF(on_error);
+    self->on_error = on_error;
+    return reinterpret_cast<PyObject*>(self);
+}
+
+void planned_dealloc(PyObject* o) {
+    PlannedCall* self = reinterpret_cast<PlannedCall*>(o);
+    PyTypeObject* type = Py_TYPE(o);
+    delete self->call;
+    Py_XDECREF(self->keep);
+    Py_XDECREF(self->on_error);
+    type->tp_free(o);
+}
+
+PyTypeObject planned_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_dispatch", "Native calls of compiled modules.", -1, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__dispatch(void) {
+    planned_type.tp_name = "daceml_b200._dispatch.PlannedCall";
+    planned_type.tp_basicsize = sizeof(PlannedCall);
+    planned_type.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_VECTORCALL;
+    planned_type.tp_new = planned_new;
+    planned_type.tp_dealloc = planned_dealloc;
+    planned_type.tp_call = PyVectorcall_Call;
+    planned_type.tp_vectorcall_offset = offsetof(PlannedCall, vectorcall);
+    if (PyType_Ready(&planned_type) < 0) return nullptr;
+    PyObject* m = PyModule_Create(&module_def);
+    if (!m) return nullptr;
+    Py_INCREF(&planned_type);
+    if (PyModule_AddObject(m, "PlannedCall", reinterpret_cast<PyObject*>(&planned_type)) < 0) return nullptr;
+    return m;
+}

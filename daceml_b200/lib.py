@@ -242,6 +242,35 @@ class Context:
 
 _contexts = {}
 _override = threading.local()
+_overrides_active = 0  # how many use_context blocks are open, in any thread
+_overrides_lock = threading.Lock()
+
+
+def overrides_active():
+    return _overrides_active
+
+
+_dispatch = None
+
+
+def dispatch_module():
+    """The native call module (``csrc/dispatch.cpp``), or None where it was not built or does not fit the installed torch:
+    compiled modules are then called through the same steps in Python."""
+    global _dispatch
+    if _dispatch is None:
+        import importlib.machinery
+        import importlib.util
+        path = os.path.join(_HERE, "lib", "_dispatch.so")
+        try:
+            loader = importlib.machinery.ExtensionFileLoader("_dispatch", path)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_dispatch", path, loader=loader))
+            loader.exec_module(module)
+            _dispatch = module
+        except (ImportError, OSError) as e:
+            import logging
+            logging.getLogger(__name__).warning("the native call module could not be loaded (%s); build it with `python -m daceml_b200.build`", e)
+            _dispatch = False
+    return _dispatch or None
 
 
 class use_context:
@@ -253,12 +282,18 @@ class use_context:
         self.ctx = ctx
 
     def __enter__(self):
+        global _overrides_active
+        with _overrides_lock:
+            _overrides_active += 1
         self.previous = getattr(_override, "ctx", None)
         _override.ctx = self.ctx
         return self.ctx
 
     def __exit__(self, *exc):
+        global _overrides_active
         _override.ctx = self.previous
+        with _overrides_lock:
+            _overrides_active -= 1
 
 
 def get_context(device=None):

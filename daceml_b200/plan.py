@@ -128,6 +128,21 @@ class LaunchPlan:
         if handle:
             self.lib.b200ml_plan_destroy(handle)
 
+    def native_call(self, inputs, outputs, order):
+        """A native callable ``tensors -> output or tuple of outputs`` that runs this plan through the device's own context,
+        or None; it returns ``NotImplemented`` for arguments it leaves to the general path.  ``inputs`` and ``outputs`` are
+        (shape, dtype) pairs, ``order`` the position of each slot's tensor among inputs and outputs."""
+        module = L.dispatch_module()
+        if module is None:
+            return None
+        ctx = L.get_context(self._device)
+
+        def on_error(rc):
+            L.check(rc)
+
+        run = ctypes.cast(self._run, ctypes.c_void_p).value
+        return module.PlannedCall(run, self.handle.value, ctx.handle.value, self._index, inputs, outputs, order, (self, ctx), on_error)
+
     def __call__(self, *addresses):
         """Enqueues the plan on the current stream; ``addresses``: one ``data_ptr()`` per name of ``io``."""
         rc = self._run(self.handle, L.get_context(self._device).handle, self._slots(*addresses), self.n_slots,

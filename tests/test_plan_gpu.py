@@ -72,3 +72,44 @@ def test_plan_follows_a_replaced_constant():
     name = next(n for n, t in module.sdfg.constants.items() if t.numel() == 64)
     module.sdfg.constants[name] = module.sdfg.constants[name] * 2.0
     assert torch.equal(module(x), y * 2.0)
+
+
+def test_graph_replays_follow_the_callers_tensors():
+    """A module that replays a CUDA graph: tensors seen again are read in place, new values in them included; the outputs stay
+    the module's own; more tensors than the module keeps graphs for, and tensors laid out otherwise, are copied as before."""
+    torch.manual_seed(0)
+    net = LeNet()
+    x0 = torch.rand(3, 1, 32, 32).cuda()
+    eager, module = DaceModule(copy.deepcopy(net), dummy_inputs=(x0, )), DaceModule(net, dummy_inputs=(x0, ), cuda_graph=True)
+    ring = [torch.rand(3, 1, 32, 32, device="cuda") for _ in range(11)]
+    first = module(ring[0])
+    for _ in range(4):
+        for x in ring:
+            x.uniform_()
+            y = module(x)
+            assert y.data_ptr() == first.data_ptr() and torch.equal(y, eager(x))
+    wide = torch.rand(3, 1, 32, 64, device="cuda")
+    assert torch.equal(module(wide[..., ::2]), eager(wide[..., ::2].contiguous()))
+    module.static_inputs[0].copy_(ring[3])
+    assert torch.equal(module(module.static_inputs[0]), eager(ring[3]))
+
+
+def test_native_call_serves_threads_and_streams():
+    import threading
+    torch.manual_seed(0)
+    nets = [DaceModule(nn.Linear(64, 48), dummy_inputs=(torch.rand(8, 64), )) for _ in range(2)]
+    xs = [torch.rand(8, 64, device="cuda") for _ in range(2)]
+    want = [m(x).clone() for m, x in zip(nets, xs)]
+    bad = []
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(200):
+                if not torch.equal(nets[i](xs[i]), want[i]):
+                    bad.append(i)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i, )) for i in range(2)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad
