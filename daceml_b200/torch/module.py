@@ -15,7 +15,6 @@ graph over static input and output buffers.
 import collections
 import functools
 import logging
-import threading
 from typing import Callable, List, Optional, Tuple
 
 import torch
@@ -214,9 +213,9 @@ class DaceModule(nn.Module):
                 return vals[0] if len(vals) == 1 else vals
             return result
 
-        run, native, enqueue = run_general, None, None
+        run, native = run_general, None
         if torch.cuda.is_available() and not debug:
-            run, native, enqueue = self._planned_call(compiled, input_names, output_names, run_general, dummy_inputs)
+            run, native = self._planned_call(compiled, input_names, output_names, run_general, dummy_inputs)
 
         if not self.cuda_graph:
             return self._as_torch_op(run, input_names, output_names, native)
@@ -244,64 +243,18 @@ class DaceModule(nn.Module):
             return holder["out"]
 
         self.static_inputs = static_in
-        return self._as_torch_op(replay, input_names, output_names, self._direct_replays(enqueue, static_in, holder, replay) if enqueue else None)
-
-    @staticmethod
-    def _direct_replays(enqueue, static_in, holder, replay, limit=8):
-        """Replays without the copy of the inputs: a caller that comes back with the same tensors (a ring of input buffers,
-        a pool's blocks) gets a graph of its own that reads them where they are and writes the same outputs.  At most
-        ``limit`` of them, the least recently used dropped first; tensors seen for the first time, and those that are not
-        laid out like the static buffers, are copied."""
-        graphs = collections.OrderedDict()
-        specs = [(b.shape, b.dtype, b.get_device()) for b in static_in]
-        lock = threading.Lock()
-
-        def plain(*args):
-            """``replay`` from plain Python; NotImplemented where the registered operator has to see the call."""
-            if (torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() or torch._C._is_torch_function_mode_enabled()
-                    or len(args) != len(specs)):
-                return NotImplemented
-            for a, (shape, dtype, device) in zip(args, specs):
-                if type(a) is not torch.Tensor or a.get_device() != device:
-                    return NotImplemented
-                if a.dtype is not dtype or a.shape != shape or not a.is_contiguous():
-                    return replay(*args)
-            key = tuple([a.data_ptr() for a in args])
-            with lock:
-                graph = graphs.get(key, NotImplemented)
-                if graph is NotImplemented:  # first sight: remember it
-                    graphs[key] = None
-                    if len(graphs) > limit:
-                        graphs.popitem(last=False)
-                else:
-                    graphs.move_to_end(key)
-                    if graph is None and not torch.cuda.is_current_stream_capturing():
-                        graph = torch.cuda.CUDAGraph()
-                        out = holder["out"]
-                        with torch.cuda.stream(torch.cuda.Stream(static_in[0].device if static_in else None)):
-                            graph.capture_begin(capture_error_mode="thread_local")
-                            try:
-                                enqueue(args, out if isinstance(out, tuple) else (out, ))
-                            finally:
-                                graph.capture_end()
-                        graphs[key] = graph
-            if graph is None or graph is NotImplemented:
-                return replay(*args)
-            graph.replay()
-            return holder["out"]
-
-        return plain
+        return self._as_torch_op(replay, input_names, output_names)
 
     @staticmethod
     def _planned_call(compiled, input_names, output_names, general, example):
         """The module as one run of the compiled SDFG's launch plan: checks the arguments, allocates the outputs, passes
         the addresses.  ``general`` serves what the plan does not take (host or strided tensors, errors to report).  Returns
-        the call in Python, its native form (None where there is none), which answers ``NotImplemented`` instead of taking
-        the general path, and the bare launch on given outputs."""
+        the call in Python and its native form (None where there is none), which answers ``NotImplemented`` instead of
+        taking the general path."""
         tensors = {n: t for n, t in zip(input_names, example) if isinstance(t, torch.Tensor)}
         plan = compiled.launch_plan(tensors if len({t.data_ptr() for t in tensors.values()}) == len(tensors) else None)
         if plan is None or sorted(compiled.io_names()) != sorted(input_names + output_names):
-            return general, None, None
+            return general, None
         arrays, constants = compiled.sdfg.arrays, compiled.sdfg.constants
         specs = [(torch.Size(arrays[n].shape), arrays[n].dtype) for n in input_names]
         out_specs = [(torch.Size(arrays[n].shape), arrays[n].dtype) for n in output_names]
@@ -323,20 +276,15 @@ class DaceModule(nn.Module):
             plan(*(addresses if in_order else [addresses[i] for i in order]))
             return outs[0] if single else tuple(outs)
 
-        def enqueue(inputs, outs):
-            """The plan on tensors that are known to fit."""
-            addresses = [t.data_ptr() for t in inputs] + [t.data_ptr() for t in outs]
-            plan(*[addresses[i] for i in order])
-
         native = plan.native_call([(tuple(s), d) for s, d in specs], [(tuple(s), d) for s, d in out_specs], order)
         if native is None:
-            return run, None, enqueue
+            return run, None
         from daceml_b200.lib import overrides_active
 
         def run_native(*args):
             return native(*args) if constants.version == version and not overrides_active() else NotImplemented
 
-        return run, run_native, enqueue
+        return run, run_native
 
     def _as_torch_op(self, function, input_names, output_names, native=None):
         """With ``compile_torch_extension`` (the default, as in the reference) the module is called through a registered

@@ -75,8 +75,8 @@ def test_plan_follows_a_replaced_constant():
 
 
 def test_graph_replays_follow_the_callers_tensors():
-    """A module that replays a CUDA graph: tensors seen again are read in place, new values in them included; the outputs stay
-    the module's own; more tensors than the module keeps graphs for, and tensors laid out otherwise, are copied as before."""
+    """A module that replays a CUDA graph: every call reads the values its tensors hold then, whether they were seen before, are
+    new, or are laid out otherwise; the outputs stay the module's own."""
     torch.manual_seed(0)
     net = LeNet()
     x0 = torch.rand(3, 1, 32, 32).cuda()
