@@ -7,6 +7,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/core/grad_mode.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -55,9 +56,11 @@ PyObject* planned_vectorcall(PyObject* self, PyObject* const* args, size_t nargs
     if (c10::impl::TorchDispatchModeTLS::stack_len() != 0 || at::impl::torch_function_mode_enabled() || torch::jit::tracer::isTracing())
         Py_RETURN_NOTIMPLEMENTED;
     void* addr[MAX_SLOTS];
+    const bool grad = at::GradMode::is_enabled();
     for (size_t i = 0; i < n; ++i) {
         if (!THPVariable_CheckExact(args[i])) Py_RETURN_NOTIMPLEMENTED;
         const at::Tensor& t = THPVariable_Unpack(args[i]);
+        if (grad && t.requires_grad()) Py_RETURN_NOTIMPLEMENTED;  // the operator's outputs carry autograd's "not implemented" node
         const Spec& s = c.inputs[i];
         if ((t.key_set().raw_repr() & ~c.plain.raw_repr()) != 0 || !t.is_cuda() || t.get_device() != c.device || t.scalar_type() != s.dtype ||
             !t.sizes().equals(s.shape) || !t.is_contiguous())

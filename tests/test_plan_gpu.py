@@ -113,3 +113,15 @@ def test_native_call_serves_threads_and_streams():
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not bad
+
+
+def test_inputs_that_require_grad_go_through_the_operator():
+    """The registered operator marks its outputs as not differentiable only when backward is called; the native call must not
+    hand out plain tensors instead."""
+    module = DaceModule(nn.Linear(8, 8), dummy_inputs=(torch.rand(4, 8), ))
+    x = torch.rand(4, 8, device="cuda")
+    want = module(x)
+    y = module(x.clone().requires_grad_())
+    assert y.requires_grad and torch.equal(y, want) and not want.requires_grad
+    with torch.no_grad():
+        assert not module(x.clone().requires_grad_()).requires_grad
