@@ -170,6 +170,10 @@ int b200ml_ctx_create(int device, int64_t workspace_bytes, b200ml_ctx** out) {
         err = cudaMalloc(&ctx->workspace, (size_t)workspace_bytes);
         ctx->workspace_bytes = workspace_bytes;
     }
+    if (err == cudaSuccess && !(ctx->scratch = scratch_pool_create(ctx->workspace, workspace_bytes))) {
+        if (ctx->workspace) cudaFree(ctx->workspace);
+        err = cudaErrorMemoryAllocation;
+    }
     if (err != cudaSuccess) {
         if (ctx->status_dev) cudaFree(ctx->status_dev);
         delete ctx;
@@ -193,7 +197,7 @@ int b200ml_ctx_create(int device, int64_t workspace_bytes, b200ml_ctx** out) {
 int b200ml_ctx_destroy(b200ml_ctx* ctx) {
     if (!ctx) return B200ML_OK;
     DeviceGuard guard(ctx->device);
-    if (ctx->workspace) cudaFree(ctx->workspace);
+    scratch_pool_destroy(ctx->scratch);
     if (ctx->status_dev) cudaFree(ctx->status_dev);
     delete ctx;
     return B200ML_OK;

@@ -23,11 +23,16 @@ enum : int32_t {
     DEV_TIMEOUT_PEER = 7,   // a rank's all-gather kernel gave up waiting for a peer's flag
 };
 
+namespace b200ml {
+struct ScratchPool;
+}
+
 struct b200ml_ctx {
     int device = 0;
     int sm_count = 0;
-    void* workspace = nullptr;
+    void* workspace = nullptr;  // scratch memory: taken through Scratch
     int64_t workspace_bytes = 0;
+    b200ml::ScratchPool* scratch = nullptr;
     int32_t* status_dev = nullptr;  // one word in device memory
     void* encode_tiled = nullptr;   // cuTensorMapEncodeTiled, resolved through the runtime
     void* mem_get_address_range = nullptr;  // cuMemGetAddressRange, likewise
@@ -86,6 +91,23 @@ struct DeviceGuard {
         if (switched) cudaSetDevice(prev);
     }
 };
+
+// Scratch memory for the launches of one call on `stream` (scratch.cu): no other call writes it before they have run.  Lives
+// until the last of them has been made; `rc` is not B200ML_OK where there is none to be had.
+class Scratch {
+public:
+    Scratch(const b200ml_ctx* ctx, int64_t bytes, cudaStream_t stream);
+    ~Scratch();
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    int rc = B200ML_OK;
+    void* ptr = nullptr;
+
+private:
+    void* block = nullptr;
+};
+ScratchPool* scratch_pool_create(void* first, int64_t bytes);  // takes `first` over; null: out of host memory
+void scratch_pool_destroy(ScratchPool* pool);
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 

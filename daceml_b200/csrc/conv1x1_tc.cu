@@ -404,7 +404,9 @@ int conv1x1_pack(const b200ml_ctx*, const b200ml_conv_params* p, void* dst, cuda
 int conv1x1_tensor_core(const b200ml_ctx* ctx, const b200ml_conv_params* p, cudaStream_t stream) {
     const int64_t hw = p->h * p->w;
     const int npad = (int)(ceil_div(p->m, 16) * 16), kpad = (int)(ceil_div(p->c + 1, PW_KB) * PW_KB);
-    float* wsplit = static_cast<float*>(ctx->workspace);
+    const Scratch scratch(ctx, p->packed_weight ? 0 : conv1x1_pack_bytes(p), stream);
+    if (scratch.rc) return scratch.rc;
+    float* wsplit = static_cast<float*>(scratch.ptr);
     if (p->packed_weight) {  // split once by the caller
         B200ML_REQUIRE(aligned16(p->packed_weight), "conv: the packed weights must be 16-byte aligned");
         wsplit = const_cast<float*>(static_cast<const float*>(p->packed_weight));

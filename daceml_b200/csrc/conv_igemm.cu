@@ -580,7 +580,9 @@ int conv_igemm_pack(const b200ml_ctx*, const b200ml_conv_params* p, int64_t ow, 
 
 int conv_igemm(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, int64_t ow, cudaStream_t stream) {
     const IgPlan pl = ig_plan(p, ow);
-    float* wsplit = static_cast<float*>(ctx->workspace);
+    const Scratch scratch(ctx, p->packed_weight ? 0 : conv_igemm_pack_bytes(p, ow), stream);
+    if (scratch.rc) return scratch.rc;
+    float* wsplit = static_cast<float*>(scratch.ptr);
     if (p->packed_weight) {  // split once by the caller
         B200ML_REQUIRE(aligned16(p->packed_weight), "conv: the packed weights must be 16-byte aligned");
         wsplit = const_cast<float*>(static_cast<const float*>(p->packed_weight));

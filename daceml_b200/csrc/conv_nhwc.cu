@@ -511,17 +511,11 @@ int conv_impl(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, in
     B200ML_REQUIRE(!(x_nhwc || y_nhwc) || (!p->pool_sum && sizeof(T) == 2), "conv: channels-last tensors are fp16 and have no pooled output");
     B200ML_REQUIRE(!x_nhwc || (p->c % 8 == 0 && !p->gate), "conv: a channels-last X needs a multiple of 8 channels and no gate");
     B200ML_REQUIRE(!y_nhwc || p->m % 8 == 0, "conv: a channels-last Y needs a multiple of 8 channels");
-    char* ws = static_cast<char*>(ctx->workspace);
-    int64_t room = ctx->workspace_bytes;
     const T* w = static_cast<const T*>(p->packed_weight);
-    T* w_out = nullptr;
-    if (!w) {
-        const int64_t bytes = ceil_div(pack_elements<T>(p) * (int64_t)sizeof(T), 1024) * 1024;
-        if (bytes > room / 2) return fail(B200ML_ERR_WORKSPACE, "conv: the weights (%lld bytes laid out) exceed the workspace", (long long)bytes);
-        w_out = reinterpret_cast<T*>(ws);
-        w = w_out;
-        ws += bytes, room -= bytes;
-    }
+    const int64_t w_bytes = w ? 0 : ceil_div(pack_elements<T>(p) * (int64_t)sizeof(T), 1024) * 1024;
+    const int64_t room = ctx->workspace_bytes - w_bytes;
+    if (w_bytes > ctx->workspace_bytes / 2)
+        return fail(B200ML_ERR_WORKSPACE, "conv: the weights (%lld bytes laid out) exceed the workspace", (long long)w_bytes);
     // images in pieces whose channels-last copy fits the workspace
     const int64_t image = cp * p->h * p->w;
     int64_t piece = p->n;
@@ -531,6 +525,11 @@ int conv_impl(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, in
         if (fit < piece) piece = fit;
         piece = ceil_div(p->n, ceil_div(p->n, piece));
     }
+    const Scratch scratch(ctx, w_bytes + (x_nhwc ? 0 : piece * image * PARTS * (int64_t)sizeof(T)), s);
+    if (scratch.rc) return scratch.rc;
+    T* w_out = w ? nullptr : static_cast<T*>(scratch.ptr);
+    if (!w) w = w_out;
+    char* ws = static_cast<char*>(scratch.ptr) + w_bytes;
     for (int64_t n0 = 0; n0 < p->n; n0 += piece) {
         const int64_t n = p->n - n0 < piece ? p->n - n0 : piece;
         const T* x = static_cast<const T*>(p->x) + n0 * p->c * p->h * p->w;

@@ -765,7 +765,9 @@ int gemm_f32(const b200ml_ctx* ctx, const b200ml_gemm_params* p, const void* pac
         const int64_t pieces = ceil_div(p->m, fit);
         rows = ceil_div(ceil_div(p->m, pieces), FM) * FM;
     }
-    float* ws_b = static_cast<float*>(ctx->workspace);
+    const Scratch scratch(ctx, (pack_b ? b_bytes : 0) + (pack_a ? packed_bytes(rows, p->k) : 0), stream);
+    if (scratch.rc) return scratch.rc;
+    float* ws_b = static_cast<float*>(scratch.ptr);
     float* ws_a = ws_b + (pack_b ? b_bytes / 4 : 0);
     for (int64_t m0 = 0; m0 < p->m; m0 += rows) {
         b200ml_gemm_params q = *p;

@@ -261,11 +261,13 @@ int gemm_f16_layernorm(const b200ml_ctx* ctx, const b200ml_gemm_params* p, cudaS
     if (tiles_m * la.cluster * 2 <= ctx->sm_count && p->m * p->n * 4 <= ctx->workspace_bytes) {
         const SplitPlan plan = gemm_f16_split_plan(ctx, p, true);
         if (plan.bn) {
-            args.c = static_cast<__half*>(ctx->workspace);  // fp32 rows of N
+            const Scratch scratch(ctx, p->m * p->n * 4, stream);
+            if (scratch.rc) return scratch.rc;
+            args.c = static_cast<__half*>(scratch.ptr);  // fp32 rows of N
             args.ldc = p->n;
             const int rc = gemm_f16_split(ctx, p, args, plan, true, stream);
             if (rc) return rc;
-            return layernorm_f32_rows(static_cast<const float*>(ctx->workspace), la.gamma, la.beta, static_cast<__half*>(p->c), (int)p->m, (int)p->n,
+            return layernorm_f32_rows(static_cast<const float*>(scratch.ptr), la.gamma, la.beta, static_cast<__half*>(p->c), (int)p->m, (int)p->n,
                                       p->ldc, la.eps, stream);
         }
     }

@@ -579,7 +579,9 @@ int reduce_t(const b200ml_ctx* ctx, int opcode, const T* x, T* y, int64_t outer,
         if (need > ctx->workspace_bytes)
             return fail(B200ML_ERR_WORKSPACE, "reduce: needs %lld bytes of scratch, the context has %lld",
                         (long long)need, (long long)ctx->workspace_bytes);
-        float* partial = static_cast<float*>(ctx->workspace);
+        const Scratch scratch(ctx, need, stream);
+        if (scratch.rc) return scratch.rc;
+        float* partial = static_cast<float*>(scratch.ptr);
         launch_pdl(reduce_rows_kernel<T>, dim3(dim3((unsigned)outer, (unsigned)slices)), dim3(256), 0, stream, x, y, partial, reduce, slices, op);
         int rc = check_launch("reduce_rows");
         if (rc) return rc;
