@@ -68,6 +68,23 @@ def _b_is_constant(node, state, sdfg, conn="B"):
     return False
 
 
+class _Packed:
+    """A copy of constants, laid out for a kernel when the graph was built.  It stands for them only while the SDFG holds what
+    it was made from and the call is given just that: a constant may be replaced, or passed by the caller of one run."""
+
+    def __init__(self, tensor, sdfg, names):
+        self.tensor, self.constants = tensor, sdfg.constants
+        self.made_from = [(n, sdfg.constants.replaced[n]) for n in names]
+
+    def get(self, device, *used):
+        """The copy, or None; ``used``: the tensors of this call in the order of the names."""
+        c = self.constants
+        if self.tensor.device != device or any(
+                n not in c or c.replaced[n] != count or c[n].data_ptr() != t.data_ptr() for (n, count), t in zip(self.made_from, used)):
+            return None
+        return self.tensor
+
+
 def _prepacked_gemm_operand(node, state, sdfg, plan, b_layout, a_layout=0):
     """A constant fp32 B is split into its TF32 parts once, here (``b200ml_gemm_prepack``); None when there is nothing to
     prepare (no device, another type, B arrives at run time, or the product takes B as it is)."""
@@ -79,7 +96,8 @@ def _prepacked_gemm_operand(node, state, sdfg, plan, b_layout, a_layout=0):
             return None
         if not t.is_cuda:
             t = t.to(torch.device("cuda", torch.cuda.current_device()))
-        return K.gemm_prepack(t.contiguous(), n=plan["n"], k=plan["k"], m=plan["m"], b_layout=b_layout, a_layout=a_layout)
+        packed = K.gemm_prepack(t.contiguous(), n=plan["n"], k=plan["k"], m=plan["m"], b_layout=b_layout, a_layout=a_layout)
+        return None if packed is None else _Packed(packed, sdfg, [e.data.data])
     return None
 
 
@@ -110,9 +128,7 @@ def _launch_gemm(a, b, out, plan, *, b_layout=0, a_layout=0, alpha=1.0, bias=Non
         p.ln_gamma = ln[0].data_ptr() if ln[0] is not None else None
         p.ln_beta = ln[1].data_ptr() if ln[1] is not None else None
         p.ln_eps = ln[2]
-    if packed is not None and packed.device != a.device:
-        packed = None
-    K.gemm_raw(ctx, p, L.current_stream(a.device), packed)
+    K.gemm_raw(ctx, p, L.current_stream(a.device), packed.get(a.device, b) if packed is not None else None)
 
 
 @op_implementation(op="MatMul", name="b200")
@@ -609,17 +625,23 @@ def _prepacked_conv_weights(node, state, sdfg, x, strides, pads, dil, group, gat
     if _has_in(node, state, "B") and not _b_is_constant(node, state, sdfg, "B"):
         return None
     dev = torch.device("cuda", torch.cuda.current_device())  # calls on another device ignore the packed copy
-    tensors = {}
+    tensors, names = {}, []
     for conn in ("W", "B"):
         for e in state.in_edges_by_connector(node, conn):
             t = sdfg.constants[e.data.data]
             if not t.is_cuda:  # a copy for the packing kernel only; the SDFG's own constant moves with its first call
                 t = t.to(dev)
             tensors[conn] = t.contiguous()
+            names.append(e.data.data)
     w = tensors["W"]
     if w.dtype not in FLOAT_TYPES or not w.is_contiguous():
         return None
-    return K.conv_prepack(tuple(x.shape), w, bias=tensors.get("B"), strides=strides, pads=pads, dilations=dil, group=group, gate=gate)
+    packed = K.conv_prepack(tuple(x.shape), w, bias=tensors.get("B"), strides=strides, pads=pads, dilations=dil, group=group, gate=gate)
+    return None if packed is None else _Packed(packed, sdfg, names)
+
+
+def _packed_of(packed, ins):
+    return packed.get(ins["X"].device, *(ins[c] for c in ("W", "B") if c in ins)) if packed is not None else None
 
 
 @op_implementation(op="Conv", name="b200")
@@ -638,7 +660,7 @@ class B200Conv(ONNXForward):
         def run(ins, outs):
             xt = ins["X"]
             K.conv2d(xt, ins["W"], outs["Y"], bias=ins.get("B"), strides=strides, pads=pads, dilations=dil,
-                     group=group, packed_weight=packed if packed is not None and packed.device == xt.device else None)
+                     group=group, packed_weight=_packed_of(packed, ins))
 
         return KernelTasklet(node.label, run, kernels=("conv2d",))
 
@@ -699,7 +721,7 @@ class B200FusedConv(ONNXForward):
             xt = ins["X"]
             K.conv2d(xt, ins["W"], outs["Y"], bias=ins.get("B"), strides=strides, pads=pads, dilations=dil,
                      group=group, act=act, gate=ins.get("Gate"), residual=ins.get("Residual"),
-                     pool_mean=outs.get("Pool"), packed_weight=packed if packed is not None and packed.device == xt.device else None)
+                     pool_mean=outs.get("Pool"), packed_weight=_packed_of(packed, ins))
 
         return KernelTasklet(node.label, run, kernels=("conv2d",))
 

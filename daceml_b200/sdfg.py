@@ -193,10 +193,21 @@ class SDFGState:
 
 
 class _Constants(dict):
-    """Constants by name; ``version`` changes with every replacement, so that a recorded launch plan can tell."""
+    """Constants by name; ``version`` changes with every replacement, so that a recorded launch plan can tell, and
+    ``replaced`` counts those of each name, so that a copy that was made of one can tell."""
     version = 0
 
+    def __new__(cls, *args, **kwargs):
+        self = super().__new__(cls, *args, **kwargs)
+        self.replaced = collections.Counter()
+        return self
+
     def __setitem__(self, key, value):
+        self.replaced[key] += 1
+        self.move(key, value)
+
+    def move(self, key, value):
+        """The same values in another place."""
         self.version += 1
         super().__setitem__(key, value)
 
@@ -209,8 +220,8 @@ class _Constants(dict):
         return super().pop(*args)
 
     def update(self, *args, **kwargs):
-        self.version += 1
-        super().update(*args, **kwargs)
+        for key, value in dict(*args, **kwargs).items():
+            self[key] = value
 
 
 class SDFG:
@@ -330,7 +341,8 @@ class CompiledSDFG:
         """The constant's tensor on this SDFG's device (moved there on first use)."""
         t = self.sdfg.constants[name]
         if not t.is_cuda:
-            t = self.sdfg.constants[name] = t.to(self._device()).contiguous()
+            t = t.to(self._device()).contiguous()
+            self.sdfg.constants.move(name, t)
         return t
 
     def io_names(self):

@@ -125,3 +125,23 @@ def test_inputs_that_require_grad_go_through_the_operator():
     assert y.requires_grad and torch.equal(y, want) and not want.requires_grad
     with torch.no_grad():
         assert not module(x.clone().requires_grad_()).requires_grad
+
+
+@pytest.mark.parametrize("kind", ["linear", "conv fp32", "conv fp16"])
+def test_packed_weights_serve_only_the_constant_they_were_made_from(kind):
+    """A constant replaced after the build, and one passed by the caller of a single run.  Powers of two scale every sum
+    exactly; fp16 results are rounded to steps of 2^-24 where they are subnormal, so y * s is within s / 2 of them."""
+    torch.manual_seed(0)
+    dtype = torch.float16 if kind == "conv fp16" else torch.float32
+    net, shape = (nn.Linear(96, 64, bias=False), (160, 96)) if kind == "linear" else (nn.Conv2d(16, 32, 3, bias=False), (2, 16, 20, 20))
+    net = net.cuda().to(dtype)
+    x = torch.randn(shape, device="cuda", dtype=dtype)
+    module = DaceModule(net, dummy_inputs=(x, ))
+    y = module(x).clone()
+    name = next(n for n, t in module.sdfg.constants.items() if t.numel() == next(net.parameters()).numel())
+    weight = module.sdfg.constants[name]
+    given = module.compiled_function(**{module.sdfg.arg_names[0]: x, name: (weight * 2.0).contiguous()})
+    step = 2.0**-24 if dtype == torch.float16 else 0.0
+    assert (given.double() - y.double() * 2.0).abs().max() <= 1.0 * step and torch.equal(module(x), y)
+    module.sdfg.constants[name] = weight * 4.0
+    assert (module(x).double() - y.double() * 4.0).abs().max() <= 2.0 * step
