@@ -59,6 +59,9 @@ struct ConvHArgs {
     int32_t sh, sw, dh, dw, pad_top, pad_left;
     int32_t act, y_nhwc;
     int32_t* status;
+    // fp32: the operands as the caller has them, for exact_conv
+    const T *x0, *w0, *gate;
+    int32_t c, h, wd, kh;
 };
 
 __device__ __forceinline__ float h_load(const float* p) { return __ldg(p); }
@@ -82,6 +85,40 @@ __device__ __forceinline__ uint64_t conv_desc(uint32_t addr, int kcb) {
     d |= 1ull << 46;
     d |= static_cast<uint64_t>(kcb == 128 ? 2 : (kcb == 64 ? 4 : 6)) << 61;
     return d;
+}
+
+// One output by itself, for fp32 sums that come out as NaN: an infinite operand has no finite lo part to go with it, and a
+// value above the largest TF32 number rounds to infinity (see gemm_f32.cu).
+__device__ __noinline__ float exact_conv(const ConvHArgs<float>& g, int n, int m, int oh, int ow) {
+    float s = 0.0f;
+    for (int c = 0; c < g.c; ++c) {
+        const float* x = g.x0 + (static_cast<int64_t>(n) * g.c + c) * g.h * g.wd;
+        const float* w = g.w0 + (static_cast<int64_t>(m) * g.c + c) * g.kh * g.kw;
+        const float gate = g.gate ? __ldg(g.gate + static_cast<int64_t>(n) * g.c + c) : 1.0f;
+        for (int i = 0; i < g.kh; ++i) {
+            const int ih = oh * g.sh - g.pad_top + i * g.dh;
+            if (ih < 0 || ih >= g.h) continue;
+            for (int j = 0; j < g.kw; ++j) {
+                const int iw = ow * g.sw - g.pad_left + j * g.dw;
+                if (iw >= 0 && iw < g.wd) s = fmaf(__ldg(x + static_cast<int64_t>(ih) * g.wd + iw) * gate, __ldg(w + i * g.kw + j), s);
+            }
+        }
+    }
+    return s;
+}
+
+// The sums of sixteen channels from m0 on of one output pixel that have to be made again.
+template <typename T>
+__device__ __forceinline__ void repair16(const ConvHArgs<T>& g, float (&v)[16], int n, int m0, int oh, int ow) {
+    if constexpr (sizeof(T) == 4) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) sum += v[j];
+        if (sum == sum) return;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (v[j] != v[j] && m0 + j < g.m) v[j] = exact_conv(g, n, m0 + j, oh, ow);
+    }
 }
 
 // Sixteen channels from m0 on of one output pixel.
@@ -285,7 +322,10 @@ conv_nhwc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                 for (int j = 0; j < 16; ++j) v[j] = 0.0f;
             }
             if (g.split == 1) {
-                if (pix_ok) finish16(g, v, mt * BN + c, pix_nchw, pix_nhwc);
+                if (pix_ok) {
+                    repair16(g, v, pn, mt * BN + c, ph, pw);
+                    finish16(g, v, mt * BN + c, pix_nchw, pix_nhwc);
+                }
                 __syncwarp();
             } else {
 #pragma unroll
@@ -308,7 +348,10 @@ conv_nhwc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] += ptx::ld_shared_cluster_f32(partial + (c + j) * H_PART_LD + row, q);
                 }
-                if (pix_ok) finish16(g, v, mt * BN + c, pix_nchw, pix_nhwc);
+                if (pix_ok) {
+                    repair16(g, v, pn, mt * BN + c, ph, pw);
+                    finish16(g, v, mt * BN + c, pix_nchw, pix_nhwc);
+                }
             }
         }
         ptx::cluster_sync_acq_rel();  // no CTA leaves while a peer may still read its partial tile
@@ -561,6 +604,9 @@ int conv_impl(const b200ml_ctx* ctx, const b200ml_conv_params* p, int64_t oh, in
         g.pad_top = (int32_t)p->pad_top, g.pad_left = (int32_t)p->pad_left;
         g.act = p->act & (B200ML_EPI_RELU | B200ML_EPI_GELU | B200ML_EPI_SWISH);
         g.y_nhwc = y_nhwc ? 1 : 0;
+        g.x0 = static_cast<const T*>(p->x) + n0 * p->c * p->h * p->w, g.w0 = static_cast<const T*>(p->weight);
+        g.gate = p->gate ? static_cast<const T*>(p->gate) + n0 * p->c : nullptr;
+        g.c = (int32_t)p->c, g.h = (int32_t)p->h, g.wd = (int32_t)p->w, g.kh = (int32_t)p->kh;
         g.status = ctx->status_dev;
         // the pixel box that covers the output with the fewest tiles; an element stride limits its extent (256 source elements)
         int64_t best = INT64_MAX;

@@ -166,9 +166,19 @@ __device__ __forceinline__ float4 ld_cluster_v4(uint32_t local_addr, uint32_t ra
     return v;
 }
 
-// alpha, bias, activation, residual of four columns of one row, and their store.
+// One element of A.B by itself.  An infinite operand has no finite lo part to go with it (inf * lo may be NaN or cancel
+// inf * hi), and a value above the largest TF32 number rounds to infinity: sums that come out as NaN are made again this way.
+__device__ __noinline__ float exact_dot(const F32Operand<float>& a, const float* pa, const F32Operand<float>& b, const float* pb, int row, int col, int k) {
+    pa += a.mn ? row : static_cast<int64_t>(row) * a.ld;
+    pb += b.mn ? col : static_cast<int64_t>(col) * b.ld;
+    float s = 0.0f;
+    for (int i = 0; i < k; ++i) s = fmaf(__ldg(pa + (a.mn ? i * a.ld : i)), __ldg(pb + (b.mn ? i * b.ld : i)), s);
+    return s;
+}
+
+// alpha, bias, activation, residual of four columns of one row, and (where `keep`) their store.
 template <typename T>
-__device__ __forceinline__ void finish4(const F32Args<T>& g, const float4& acc, T* c, const T* res, int row, int col) {
+__device__ __forceinline__ void finish4(const F32Args<T>& g, const float4& acc, T* c, const T* res, int row, int col, bool keep) {
     const int valid = g.n - col;
     float v[4] = {g.ep.alpha * acc.x, g.ep.alpha * acc.y, g.ep.alpha * acc.z, g.ep.alpha * acc.w};
     if ((g.ep.flags & B200ML_EPI_BIAS) && g.bias) {
@@ -183,7 +193,7 @@ __device__ __forceinline__ void finish4(const F32Args<T>& g, const float4& acc, 
         v[0] = fmaf(g.ep.residual_scale, q.x, v[0]), v[1] = fmaf(g.ep.residual_scale, q.y, v[1]);
         v[2] = fmaf(g.ep.residual_scale, q.z, v[2]), v[3] = fmaf(g.ep.residual_scale, q.w, v[3]);
     }
-    store4(c + static_cast<int64_t>(row) * g.ldc + col, g.c_vec, valid, v);
+    if (keep) store4(c + static_cast<int64_t>(row) * g.ldc + col, g.c_vec, valid, v);
 }
 
 template <typename T, int BN, bool PACKED_A, bool PACKED_B>
@@ -412,21 +422,42 @@ __global__ void __launch_bounds__(F_THREADS, 1) gemm_f32_kernel(const F32Args<T>
         const T* res = g.residual ? g.residual + bo * g.r_so + bi * g.r_si : nullptr;
         const uint32_t part_addr = ptx::smem_u32(smem);
         if (col < g.n) {
+            auto summed = [&](int rt) {
+                const uint32_t at = part_addr + (rt * S::PART_LD + (t % C4) * 4) * 4;
+                if (g.split == 1) return convtc::ld_shared_v4(at);
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                for (int q = 0; q < g.split; ++q) {  // rank order: the same sum on every run
+                    const float4 w = ld_cluster_v4(at, q);
+                    v.x += w.x, v.y += w.y, v.z += w.z, v.w += w.w;
+                }
+                return v;
+            };
+            bool again = false;
             for (int r = t / C4; r < share; r += ROWS_PER_PASS) {
                 const int rt = rank * share + r, row = m0 + rt;
                 if (row >= g.m) break;
-                const uint32_t at = part_addr + (rt * S::PART_LD + (t % C4) * 4) * 4;
-                float4 v;
-                if (g.split == 1) {
-                    v = convtc::ld_shared_v4(at);
-                } else {
-                    v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    for (int q = 0; q < g.split; ++q) {  // rank order: the same sum on every run
-                        const float4 w = ld_cluster_v4(at, q);
-                        v.x += w.x, v.y += w.y, v.z += w.z, v.w += w.w;
+                const float4 v = summed(rt);
+                const float sum = (v.x + v.y) + (v.z + v.w);
+                const bool keep = PARTS == 1 || sum == sum;  // else a NaN among them, or infinities of both signs: below
+                again |= !keep;
+                finish4(g, v, c, res, row, col, keep);
+            }
+            if constexpr (PARTS == 2) {
+                if (again) {
+                    const float *pa = g.a.p + bo * g.a.so + bi * g.a.si, *pb = g.b.p + bo * g.b.so + bi * g.b.si;
+                    for (int r = t / C4; r < share; r += ROWS_PER_PASS) {
+                        const int rt = rank * share + r, row = m0 + rt;
+                        if (row >= g.m) break;
+                        float4 v = summed(rt);
+                        const float sum = (v.x + v.y) + (v.z + v.w);
+                        if (sum == sum) continue;
+                        if (v.x != v.x) v.x = exact_dot(g.a, pa, g.b, pb, row, col, g.k);
+                        if (v.y != v.y && col + 1 < g.n) v.y = exact_dot(g.a, pa, g.b, pb, row, col + 1, g.k);
+                        if (v.z != v.z && col + 2 < g.n) v.z = exact_dot(g.a, pa, g.b, pb, row, col + 2, g.k);
+                        if (v.w != v.w && col + 3 < g.n) v.w = exact_dot(g.a, pa, g.b, pb, row, col + 3, g.k);
+                        finish4(g, v, c, res, row, col, true);
                     }
                 }
-                finish4(g, v, c, res, row, col);
             }
         }
     }

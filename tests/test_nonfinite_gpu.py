@@ -1,0 +1,62 @@
+"""Infinite, NaN and very large fp32 operands: products that run as 3 x TF32 give what the sum in fp32 gives."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from daceml_b200 import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+BIG = 3.4028234e38  # rounds to infinity at TF32's mantissa
+
+
+def _plant(x):
+    """Infinities, a NaN and a value above the largest TF32 number, each in a row (image) of its own."""
+    flat = x.reshape(x.shape[0], -1)
+    flat[0, 1], flat[1, 2], flat[2, 3], flat[3, 4] = float("inf"), -float("inf"), float("nan"), BIG
+    return x
+
+
+def _check(got, want):
+    """``want`` in 64 bits; finite results to 1e-5 of the largest one of their row, which the planted values dominate."""
+    got, want = got.double().flatten(1), want.flatten(1)
+    assert torch.equal(got.isnan(), want.isnan())
+    inf = want.isinf()
+    assert torch.equal(got[inf], want[inf]) and not got[~inf & ~want.isnan()].isinf().any()
+    scale = want.masked_fill(inf | want.isnan(), 0.0).abs().amax(1, keepdim=True)
+    err = torch.where(inf | want.isnan(), torch.zeros_like(want), (got - want).abs())
+    assert (err <= 1e-5 * scale).all()
+
+
+@pytest.mark.parametrize("m,n,k,packed", [(40, 24, 70, False), (130, 130, 64, True), (700, 520, 96, False), (2500, 1100, 40, True), (257, 33, 700, True)])
+def test_products(m, n, k, packed):
+    torch.manual_seed(0)
+    a, b = _plant(torch.randn(m, k)).cuda(), (torch.randn(n, k) * 0.01).cuda()
+    b[0] = torch.where(b[0] == 0, b[0] + 0.5, b[0])
+    out = torch.empty(m, n, device="cuda")
+    if packed:
+        import ctypes
+        from daceml_b200 import lib as L
+        p = L.GemmParams()
+        p.dtype, p.b_layout, p.m, p.n, p.k, p.batch_outer, p.batch_inner = L.F32, 1, m, n, k, 1, 1
+        p.lda, p.ldb, p.ldc, p.alpha, p.bias_scale, p.residual_scale = k, k, n, 1.0, 1.0, 1.0
+        p.a, p.b, p.c = a.data_ptr(), b.data_ptr(), out.data_ptr()
+        K.gemm_raw(L.get_context(0), p, L.current_stream(), K.gemm_prepack(b, n=n, k=k, m=m, b_layout=1))
+    else:
+        K.gemm(a, b, out, b_layout=1)
+    want = a.double() @ b.double().T
+    _check(out, want)
+
+
+@pytest.mark.parametrize("n,c,m,size,kernel,stride", [(4, 24, 32, 20, 3, 1), (4, 8, 70, 9, 3, 2), (5, 64, 16, 12, 1, 1), (4, 256, 64, 7, 3, 1)])
+def test_convolutions(n, c, m, size, kernel, stride):
+    torch.manual_seed(0)
+    x, w = _plant(torch.randn(n, c, size, size)).cuda(), (torch.randn(m, c, kernel, kernel) * 0.01).cuda()
+    pad = kernel // 2
+    out = torch.empty(n, m, (size + 2 * pad - kernel) // stride + 1, (size + 2 * pad - kernel) // stride + 1, device="cuda")
+    K.conv2d(x, w, out, strides=(stride, stride), pads=(pad, ) * 4)
+    # the window sum by hand: a library convolution may use another algorithm, for which inf * 0 is no term of the sum
+    cols = F.unfold(x.double().cpu(), kernel, padding=0 if pad == 0 else pad, stride=stride)
+    mask = F.unfold(torch.ones(1, c, size, size, dtype=torch.float64), kernel, padding=pad, stride=stride) > 0
+    terms = torch.where(mask[:, None], cols[:, None] * w.double().cpu().flatten(1)[None, :, :, None], torch.zeros((), dtype=torch.float64))
+    _check(out.cpu(), terms.sum(2).view(out.shape))
