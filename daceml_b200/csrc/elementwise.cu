@@ -436,23 +436,27 @@ int binary_t(const b200ml_ctx* ctx, int op, const T* a, const T* b, T* y, int ra
     int64_t n = 1;
     for (int d = 0; d < rank; ++d) n *= shape[d];
     if (n == 0) return B200ML_OK;
-    // Classify each operand: dense (contiguous strides), scalar (all zero), or a vector on the
-    // last axis (stride 1 there, zero elsewhere).
-    auto classify = [&](const int64_t* st) {
-        bool dense = true, scalar = true, lastvec = rank >= 1;
+    // Classify each operand: dense (contiguous strides, 0), scalar (all zero, 1), or periodic (2): contiguous over the last axes,
+    // zero strides in front of them - a row vector, or a block such as a position embedding added to every sample
+    // (32 x 128 x 768 fp16 plus 128 x 768: 24.6 us on the general kernel, which divides for every element, 7.5 in packets).
+    int64_t period_a = 1, period_b = 1;
+    auto classify = [&](const int64_t* st, int64_t* period) {
+        bool dense = true, scalar = true, periodic = true, repeats = false;
         int64_t expect = 1;
+        *period = 1;
         for (int d = rank - 1; d >= 0; --d) {
             if (shape[d] != 1) {
                 if (st[d] != expect) dense = false;
                 if (st[d] != 0) scalar = false;
-                if (d == rank - 1 ? st[d] != 1 : st[d] != 0) lastvec = false;
+                if (st[d] == 0) repeats = true;
+                else if (repeats || st[d] != expect) periodic = false;
+                if (!repeats) *period *= shape[d];
             }
             expect *= shape[d];
         }
-        return dense ? 0 : (scalar ? 1 : (lastvec ? 2 : 3));
+        return dense ? 0 : (scalar ? 1 : (periodic ? 2 : 3));
     };
-    const int ca = rank == 0 ? 0 : classify(as), cb = rank == 0 ? 0 : classify(bs);
-    const int64_t last = rank ? shape[rank - 1] : 1;
+    const int ca = rank == 0 ? 0 : classify(as, &period_a), cb = rank == 0 ? 0 : classify(bs, &period_b);
     const bool vec_ok = n % V == 0 && aligned16(y);
     if (vec_ok && ca == 0 && cb == 0 && aligned16(a) && aligned16(b) && op <= B200ML_BIN_DIV) {
         const unsigned grid = grid_for((n / V + 1) / 2, ctx->sm_count);
@@ -464,12 +468,12 @@ int binary_t(const b200ml_ctx* ctx, int op, const T* a, const T* b, T* y, int ra
         }
         return check_launch("binary_same");
     }
-    if (vec_ok && ca == 0 && aligned16(a) && (cb == 0 ? aligned16(b) : cb == 1 ? true : (cb == 2 && last % V == 0 && aligned16(b)))) {
-        launch_pdl(binary_fast_kernel<T>, dim3(grid_for(n / V, ctx->sm_count)), dim3(256), 0, s, a, b, y, n, op, cb, last, 0);
+    if (vec_ok && ca == 0 && aligned16(a) && (cb == 0 ? aligned16(b) : cb == 1 ? true : (cb == 2 && period_b % V == 0 && aligned16(b)))) {
+        launch_pdl(binary_fast_kernel<T>, dim3(grid_for(n / V, ctx->sm_count)), dim3(256), 0, s, a, b, y, n, op, cb, period_b, 0);
         return check_launch("binary_fast");
     }
-    if (vec_ok && cb == 0 && aligned16(b) && (ca == 1 || (ca == 2 && last % V == 0 && aligned16(a)))) {
-        launch_pdl(binary_fast_kernel<T>, dim3(grid_for(n / V, ctx->sm_count)), dim3(256), 0, s, b, a, y, n, op, ca, last, 1);
+    if (vec_ok && cb == 0 && aligned16(b) && (ca == 1 || (ca == 2 && period_a % V == 0 && aligned16(a)))) {
+        launch_pdl(binary_fast_kernel<T>, dim3(grid_for(n / V, ctx->sm_count)), dim3(256), 0, s, b, a, y, n, op, ca, period_a, 1);
         return check_launch("binary_fast");
     }
     BcastArgs g{};

@@ -713,3 +713,24 @@ def test_conv_prepacked_weights(rng):
     ws = dev(rng.standard_normal((16, 3, 3, 3)).astype(np.float32))
     assert K.conv_prepack((32, 3, 64, 64), ws, strides=(2, 2)) is None                         # 27 terms: the direct kernel
     status_ok()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("shape,other", [((4, 6, 16), (6, 16)), ((4, 6, 16), (1, 6, 16)), ((3, 5, 1, 8), (5, 1, 8)), ((2, 3, 4, 8), (1, 3, 1, 8)),
+                                         ((5, 3, 7), (3, 7)), ((2, 6, 4), (6, 1)), ((32, 128, 768), (128, 768)), ((7, 2, 4), (2, 4))])
+def test_binary_periodic_operand(dtype, shape, other):
+    """A block that repeats over the leading axes (packets where its size allows), on either side; division rounds once."""
+    torch.manual_seed(0)
+    def away_from_zero(size):
+        return ((torch.rand(size, device="cuda") + 0.5) * (torch.rand(size, device="cuda") - 0.5).sign()).to(dtype)
+
+    a, b = away_from_zero(shape), away_from_zero(other)
+    b = torch.where(b == 0, torch.ones_like(b), b)
+    a = torch.where(a == 0, torch.ones_like(a), a)
+    for op, fn in ((L.BIN_ADD, torch.add), (L.BIN_SUB, torch.sub), (L.BIN_DIV, torch.div)):
+        for x, y in ((a, b), (b, a)):
+            out = torch.empty(shape, device="cuda", dtype=dtype)
+            K.binary(x, y, out, op)
+            want = fn(x.double(), y.double())
+            eps = 2.0**-11 if dtype == torch.float16 else 2.0**-22
+            assert ((out.double() - want).abs() <= eps * want.abs() + 2.0**-25).all()
