@@ -36,14 +36,15 @@ constexpr int F_NACC = 4;
 constexpr int F_THREADS = 320;  // warp 0: MMA; warps 1-8: producers, then epilogue; warp 9: copies of a packed B
 constexpr int F_PACK_ROWS = 32; // packed B: rows are padded to a multiple of this
 
-template <typename T, int BN>
+template <typename T, int BN, int CTAS>
 struct F32Smem {
     static constexpr int PARTS = sizeof(T) == 4 ? 2 : 1;  // hi and lo; fp16 values have no lo part
     static constexpr int A_BYTES = FM * FK * 4, B_BYTES = BN * FK * 4;
     static constexpr int STAGE_BYTES = PARTS * (A_BYTES + B_BYTES);
-    // As many as fit beside the barriers; more than half of an SM's shared memory in every case, so that no two CTAs - of one
-    // cluster, waiting for one another - can share an SM and wait for each other's tensor memory.
-    static constexpr int STAGES = BN == 128 ? 6 / PARTS : (PARTS == 1 ? 8 : 4);
+    // One CTA on an SM: as many as fit beside the barriers; more than half of an SM's shared memory in every case, so that no
+    // two CTAs - of one cluster, waiting for one another - can share an SM and wait for each other's tensor memory.  Two CTAs
+    // (no clusters; BN of 64 at most, so that the tensor memory serves both): half as many.
+    static constexpr int STAGES = (BN == 128 ? 6 / PARTS : (PARTS == 1 ? 8 : 4)) / CTAS;
     static constexpr int PART_LD = BN + 4;  // floats between rows of the parked tile: 16-byte rows, no bank conflicts
     static constexpr int TOTAL = STAGES * STAGE_BYTES + 256 + 1024;
     static_assert(FM * PART_LD * 4 <= STAGES * STAGE_BYTES, "the parked tile lies over the pipeline stages");
@@ -196,9 +197,9 @@ __device__ __forceinline__ void finish4(const F32Args<T>& g, const float4& acc, 
     if (keep) store4(c + static_cast<int64_t>(row) * g.ldc + col, g.c_vec, valid, v);
 }
 
-template <typename T, int BN, bool PACKED_A, bool PACKED_B>
-__global__ void __launch_bounds__(F_THREADS, 1) gemm_f32_kernel(const F32Args<T> g) {
-    using S = F32Smem<T, BN>;
+template <typename T, int BN, bool PACKED_A, bool PACKED_B, int CTAS>
+__global__ void __launch_bounds__(F_THREADS, CTAS) gemm_f32_kernel(const F32Args<T> g) {
+    using S = F32Smem<T, BN, CTAS>;
     constexpr int STAGES = S::STAGES, PARTS = S::PARTS;
     constexpr uint32_t TMEM_COLS = F_NACC * BN;
     extern __shared__ uint8_t smem_raw[];
@@ -664,10 +665,10 @@ bool rows_applies(const b200ml_gemm_params* p) {
     return p->a_layout == 0 && p->b_layout == 1 && p->m <= 32 && p->batch_outer * p->batch_inner <= 65535;
 }
 
-template <typename T, int BN, bool PACKED_A, bool PACKED_B>
+template <typename T, int BN, bool PACKED_A, bool PACKED_B, int CTAS = 1>
 int launch_f32(const b200ml_ctx* ctx, F32Args<T>& g, int64_t tiles, int split, cudaStream_t stream) {
-    using S = F32Smem<T, BN>;
-    auto kernel = gemm_f32_kernel<T, BN, PACKED_A, PACKED_B>;
+    using S = F32Smem<T, BN, CTAS>;
+    auto kernel = gemm_f32_kernel<T, BN, PACKED_A, PACKED_B, CTAS>;
     static bool configured[64] = {};  // per instantiation and device
     if (!configured[ctx->device & 63]) {
         B200ML_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
@@ -736,6 +737,11 @@ int gemm_f32_impl(const b200ml_ctx* ctx, const b200ml_gemm_params* p, const floa
     // Tile width: narrow outputs get narrow tiles; so do products that would leave most SMs idle even with K split eight ways.
     int bn = p->n <= 32 ? 32 : (p->n <= 64 ? 64 : 128);
     if (!packed_a && bn == 128 && g.tiles_m * ceil_div(p->n, 128) * batches * 8 <= ctx->sm_count) bn = 64;
+    // More tiles than SMs whose reduction is short (the scores of an attention head: K = 64) or whose width is 64 or less (the
+    // product with V): a tile is mostly latency - first loads, hand-overs, epilogue - and two CTAs on an SM hide each other's.
+    // us, one -> two: 96 x 512 x 512 x 64 (128 columns -> 64) 116.4 -> 104.0, 64 x 300 x 300 x 64 42.0 -> 34.2; 96 x 512 x 64 x 512
+    // 72.2 -> 61.8.  At K = 128 the narrower tiles' second load of A costs what is won (16 x 512 x 512: 27.9 -> 28.7).
+    if (!packed_a && !packed_b && bn == 128 && num_kb <= 2 && g.tiles_m * ceil_div(p->n, 64) * batches > 2 * ctx->sm_count) bn = 64;
     g.tiles_n = (int32_t)ceil_div(p->n, bn);
     const int64_t tiles = (int64_t)g.tiles_m * g.tiles_n * batches;
     B200ML_REQUIRE(tiles < (1ll << 27), "gemm: too many tiles");
@@ -752,6 +758,7 @@ int gemm_f32_impl(const b200ml_ctx* ctx, const b200ml_gemm_params* p, const floa
             }
         }
     }
+    if (bn == 64 && tiles > ctx->sm_count) return launch_f32<T, 64, false, false, 2>(ctx, g, tiles, split, stream);
     switch (bn) {
         case 32: return launch_f32<T, 32, false, false>(ctx, g, tiles, split, stream);
         case 64: return launch_f32<T, 64, false, false>(ctx, g, tiles, split, stream);
