@@ -1,4 +1,4 @@
-// The epilogue of the GEMM + LayerNorm kernels: everything after the last product of a CTA's 128 x 256 tile.
+// The epilogue of the GEMM + LayerNorm kernels: everything after the last product of a CTA's 128 x BN tile (BN of 256, 192 or 128).
 //   pass A   finish the GEMM epilogue in fp32 (alpha, bias, ReLU, residual), park the values in TMEM, accumulate
 //            the row's sum and sum of squares;
 //   exchange the CTAs that hold the other columns of the same rows read each other's per-row sums through
@@ -17,11 +17,17 @@ struct LnArgs {
     const __half* gamma;
     const __half* beta;
     float eps;
-    int32_t cluster;  // CTAs (or CTA pairs) per row block = N / 256
 };
 
-// Where the sixteen 32-row x 64-column residual tiles of a CTA sit in shared memory (tile t: epilogue warp t / 2,
-// its 64-column half t % 2): the first `split` tiles in one freed pipeline stage, the rest in the next.
+// How the columns of a tile are dealt to the two epilogue warps of a TMEM lane quarter: whole pieces of 64 (one staging tile).
+template <int BN>
+struct LnCols {
+    static constexpr int H0 = BN >= 192 ? 128 : 64, H1 = BN - H0;
+    static constexpr int RES_TILES = 4 * (BN / 64);  // 32-row x 64-column tiles of the residual
+};
+
+// Where the 32-row x 64-column residual tiles of a CTA sit in shared memory (the first column half's warps in order, then the
+// second's, each with its pieces of 64 columns): the first `split` tiles in one freed pipeline stage, the rest in the next.
 struct ResidualTiles {
     uint8_t* first;
     uint8_t* second;
@@ -32,7 +38,7 @@ struct ResidualTiles {
 
 // peers: the NPEERS cluster ranks peer_first + i * peer_step hold the same rows.  G: 32-column chunks in flight per
 // warp (2 needs about 168 registers per thread, 1 about 96).
-template <int NPEERS, int G>
+template <int BN, int NPEERS, int G>
 __device__ __forceinline__ void layernorm_epilogue(const LnArgs& la, const CUtensorMap* tmap_c, uint32_t tmem_base,
                                                    uint8_t* out_stage, const ResidualTiles& res, float* red, float* stats,
                                                    uint64_t* tmem_full_bar, uint64_t* res_full_bar, int m0, int n0,
@@ -41,10 +47,13 @@ __device__ __forceinline__ void layernorm_epilogue(const LnArgs& la, const CUten
     bool epi_ok = true;
     const bool is_epi = warp >= 2;
     const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;           // columns [half * 128, half * 128 + 128) of this CTA's tile
+    const int half = (warp - 2) >> 2;           // the first H0 columns of this CTA's tile, or the H1 behind them
+    constexpr int H0 = LnCols<BN>::H0, H1 = LnCols<BN>::H1;
+    const int chunks = (half ? H1 : H0) / 32;
+    const int res_first = half ? 4 * (H0 / 64) + (warp - 6) * (H1 / 64) : (warp - 2) * (H0 / 64);
     const int row_in_tile = quarter * 32 + lane;
-    const uint32_t t_base = tmem_base + half * 128 + (static_cast<uint32_t>(quarter * 32) << 16);
-    const int col_base = n0 + half * 128;
+    const uint32_t t_base = tmem_base + half * H0 + (static_cast<uint32_t>(quarter * 32) << 16);
+    const int col_base = n0 + half * H0;
     const float inv_n = 1.0f / static_cast<float>(args.n);
     float mean = 0.0f, rstd = 0.0f;
 
@@ -65,7 +74,7 @@ __device__ __forceinline__ void layernorm_epilogue(const LnArgs& la, const CUten
             }
             const bool relu = (args.epilogue & B200ML_EPI_RELU) != 0;
 #pragma unroll 1
-            for (int c = 0; c < 4; c += G) {
+            for (int c = 0; c < chunks; c += G) {
                 uint32_t r[G][32];
                 uint4 rb[G][4], rr[G][4];
 #pragma unroll
@@ -78,7 +87,7 @@ __device__ __forceinline__ void layernorm_epilogue(const LnArgs& la, const CUten
                         for (int g = 0; g < 4; ++g) rb[u][g] = __ldg(reinterpret_cast<const uint4*>(args.bias + col0 + g * 8));
                     }
                     if (has_res) {
-                        const uint8_t* tile_row = res.tile((warp - 2) * 2 + ((c + u) >> 1)) + lane * 128;
+                        const uint8_t* tile_row = res.tile(res_first + ((c + u) >> 1)) + lane * 128;
 #pragma unroll
                         for (int g = 0; g < 4; ++g)
                             rr[u][g] = *reinterpret_cast<const uint4*>(tile_row + (((((c + u) & 1) * 4 + g) ^ (lane & 7)) << 4));
@@ -136,7 +145,7 @@ __device__ __forceinline__ void layernorm_epilogue(const LnArgs& la, const CUten
             uint8_t* stage_tile = out_stage + (warp - 2) * 4096;
             uint8_t* stage_row = stage_tile + lane * 128;
 #pragma unroll 1
-            for (int c = 0; c < 4; c += G) {
+            for (int c = 0; c < chunks; c += G) {
                 uint32_t r[G][32];
                 uint4 rg[G][4], rb[G][4];
 #pragma unroll

@@ -59,3 +59,26 @@ def test_layernorm_behind_a_gemm(m, n, k):
     assert bool((err <= bound).all()), "worst error / bound %.3g" % float((err / bound).max())
     assert bool((guard[m:] == 7.0).all())
     assert L.get_context(0).device_status() == 0
+
+
+@pytest.mark.parametrize("b_layout", [0, 1])
+@pytest.mark.parametrize("with_res", [True, False])
+@pytest.mark.parametrize("m, n, k", [(6000, 256, 264), (4000, 512, 200), (9000, 512, 64), (19300, 256, 72), (4000, 768, 648), (6000, 768, 72), (4001, 512, 2048)])
+def test_fused_layernorm_tile_widths(m, n, k, with_res, b_layout):
+    """Clusters of two and four CTAs on tiles of 128 columns, four on 192, one to three on 256; ragged last row block."""
+    gen = torch.Generator("cuda").manual_seed(7)
+
+    def rand(*s, scale=1.0):
+        return (torch.randn(*s, device="cuda", generator=gen) * scale).half()
+
+    a, b, bias, gamma, beta = rand(m, k), rand(n, k, scale=k**-0.5), rand(n), rand(n), rand(n)
+    res = rand(m, n) if with_res else None
+    pre = a.double() @ b.double().t() + bias.double() + (res.double() if with_res else 0.0)
+    ref = torch.nn.functional.layer_norm(pre, (n, ), gamma.double(), beta.double(), 1e-12)
+    guard = torch.full((m + 2, n), 7.0, dtype=torch.float16, device="cuda")
+    K.gemm(a, b if b_layout else b.t().contiguous(), guard[:m], b_layout=b_layout, bias=bias, residual=res, ln=(gamma, beta, 1e-12))
+    err = (guard[:m].double() - ref).abs()
+    bound = 2.0**-10 * ref.abs() + 2e-5 * (1.0 + gamma.double().abs()) + 1e-5  # as above
+    assert bool((err <= bound).all()), "worst error / bound %.3g" % float((err / bound).max())
+    assert bool((guard[m:] == 7.0).all())
+    assert L.get_context(0).device_status() == 0
