@@ -673,7 +673,7 @@ def alias_reshapes(sdfg, state):
 @_each_state
 def keep_channels_last(sdfg, state):
     """A transient written by one fp16 convolution and read by others only as their X keeps its values channels-last, the
-    order the tensor-core kernel reads (``csrc/conv_f16.cu``): no turn between the two.  Run last, before expansion."""
+    order the tensor-core kernel reads (``csrc/conv_nhwc.cu``): no turn between the two.  Run last, before expansion."""
     from daceml_b200 import kernels as K
 
     if not torch.cuda.is_available():
